@@ -14,30 +14,26 @@
 //                     tiles in a single persistent launch after a range pass; used where no
 //                     scratch for the slots exists (fz_compress_noalloc).
 //
-// Work decomposition: one warp owns one 2048-code shuffle block.  The warp computes its
-// codes from the floats (halo rows come from L2), stages them in 4 KiB of shared memory,
-// transposes 32x32 bit tiles in registers, derives the chunk flags with 8 ballots (which
-// are exactly the 8 bitmap words of the block) and writes its non-zero chunks with
-// 128-bit stores.
+// Work decomposition: one warp owns one 2048-code shuffle block.  Its codes come from the
+// CTA's staged quantised values (fz_encode.cuh) or, where magnitudes or row widths do not
+// allow that, from the floats (compute_block: halo rows come from L2, codes staged in 4 KiB of
+// shared memory).  The warp transposes 32x32 bit tiles in registers, derives the chunk flags
+// with 8 ballots (which are exactly the 8 bitmap words of the block) and writes its non-zero
+// chunks with 128-bit stores.
 #include <algorithm>
 #include <atomic>
 
+#include "fz_encode.cuh"
 #include "fz_internal.h"
 
-#ifndef FZ_ENCODE_RING
-#define FZ_ENCODE_RING 4
-#endif
 #ifndef FZ_RANGE_VEC
 #define FZ_RANGE_VEC 8
-#endif
-#ifndef FZ_ENCODE_CTAS
-#define FZ_ENCODE_CTAS 3
 #endif
 #ifndef FZ_BLOCK3D_UNROLL
 #define FZ_BLOCK3D_UNROLL 2
 #endif
-#ifndef FZ_ENCODE_CTAS_2D
-#define FZ_ENCODE_CTAS_2D 5
+#ifndef FZ_ENCODE_CTAS
+#define FZ_ENCODE_CTAS 4
 #endif
 #ifndef FZ_RANGE_CTAS
 #define FZ_RANGE_CTAS 5
@@ -295,138 +291,6 @@ __device__ __forceinline__ void block1d(const float* __restrict__ in, uint32_t b
             if ((lane & 7u) == 0) signw[(base >> 5) + it * 4 + (lane >> 3)] = sv;
         }
         v = vn;
-        e0 += 128;
-    }
-    ovf |= (!(amax0 < 32768.0f) || !(amax1 < 65536.0f)) ? 1u : 0u;
-}
-
-// ------------------------------------------------- asynchronous row ring --
-// The whole-block paths below keep kRing group rows of input in flight per warp without
-// holding them in registers: every lane copies its own 16-byte pieces (its 4 elements of
-// the centre row and of the north row) into a per-warp ring in shared memory with
-// cp.async, kRing group rows ahead, and waits only for its own copies (cp.async.wait_group),
-// so no lane waits for another.  A north row outside the element's tile is zero-filled
-// (source size 0) instead of read.
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait()
-{
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// block2d with the ring: the same float expressions, positions and carried west values;
-// group row it's inputs come from ring slot it % kRing, refilled with group row it + kRing
-// once they have been used.
-template <int kRing>
-__device__ __forceinline__ void block2d_ring(const float* __restrict__ in, const Geo& g, uint32_t base, float r,
-                                             uint32_t lane, uint32_t* sm, float4* ring, uint32_t& ovf)
-{
-    static_assert(kRing >= 2 && 4 % kRing == 0, "slot of an unrolled row is a constant");
-    uint32_t       e0 = base + lane * 4;
-    uint32_t       row0 = fdiv(e0, g.dx), col0 = e0 - row0 * g.x;  // group row being computed
-    uint32_t       ei = e0, rowi = row0, coli = col0;              // group row being fetched
-    const uint32_t rs = (uint32_t)__cvta_generic_to_shared(ring) + lane * 16;
-#pragma unroll
-    for (int k = 0; k < kRing; ++k) {
-        const bool nin = (rowi & 15u) != 0;
-        cp_async16(rs + k * 1024, in + ei, 16);
-        cp_async16(rs + k * 1024 + 512, nin ? in + (ei - g.x) : in + ei, nin ? 16u : 0u);
-        cp_async_commit();
-        advance128(g, ei, rowi, coli);
-        ei += 128;
-    }
-    // t = c - n of element base-1, the west neighbour of lane 0's first group
-    float carry = 0.0f;
-    if (lane == 0 && (col0 & 15u))
-        carry = __fsub_rn(pq(__ldg(in + e0 - 1), r), (row0 & 15u) ? pq(__ldg(in + e0 - 1 - g.x), r) : 0.0f);
-    SwzRot         so(lane);
-    const uint32_t prev = (lane + 31u) & 31u;
-    float          amax = 0.0f;
-#pragma unroll 4
-    for (uint32_t it = 0; it < 16; ++it) {
-        cp_async_wait<kRing - 1>();  // this lane's copies of group row it have landed
-        const float4* slot = ring + (it % kRing) * 64 + lane;
-        const float4  v0 = slot[0], u0 = slot[32];
-        const bool    cin = (col0 & 15u) != 0;
-        float         t[4];
-        t[0] = __fsub_rn(pq(v0.x, r), pq(u0.x, r));
-        t[1] = __fsub_rn(pq(v0.y, r), pq(u0.y, r));
-        t[2] = __fsub_rn(pq(v0.z, r), pq(u0.z, r));
-        t[3] = __fsub_rn(pq(v0.w, r), pq(u0.w, r));
-        const float rot = __shfl_sync(kFull, t[3], prev);
-        const float tw  = cin ? (lane ? rot : carry) : 0.0f;
-        carry           = rot;
-        float d[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) d[j] = __fsub_rn(t[j], j ? t[j - 1] : tw);
-        amax = fmax3_nan(amax, fabsf(d[0]), fabsf(d[1]));
-        amax = fmax3_nan(amax, fabsf(d[2]), fabsf(d[3]));
-        *reinterpret_cast<uint2*>(sm + it * 64 + so.x0) =
-            make_uint2(pack_signed_pair(d[0], d[1]), pack_signed_pair(d[2], d[3]));
-        so.next();
-        if (it + kRing < 16) {  // the slot's values are in registers and used: refill it
-            const bool     nin = (rowi & 15u) != 0;
-            const uint32_t dst = rs + (it % kRing) * 1024;
-            cp_async16(dst, in + ei, 16);
-            cp_async16(dst + 512, nin ? in + (ei - g.x) : in + ei, nin ? 16u : 0u);
-            advance128(g, ei, rowi, coli);
-            ei += 128;
-        }
-        cp_async_commit();  // (empty in the last rows: keeps the group count per row)
-        advance128(g, e0, row0, col0);
-        e0 += 128;
-    }
-    ovf |= !(amax < 32768.0f) ? 1u : 0u;
-}
-
-// block1d with the ring (centre rows only).
-template <int kRing>
-__device__ __forceinline__ void block1d_ring(const float* __restrict__ in, uint32_t base, float r, uint32_t lane,
-                                             uint32_t* sm, uint32_t* signw, float4* ring, uint32_t& ovf)
-{
-    static_assert(kRing >= 2 && 4 % kRing == 0, "slot of an unrolled row is a constant");
-    uint32_t       e0 = base + lane * 4;
-    const uint32_t rs = (uint32_t)__cvta_generic_to_shared(ring) + lane * 16;
-#pragma unroll
-    for (int k = 0; k < kRing; ++k) {
-        cp_async16(rs + k * 1024, in + e0 + 128 * k, 16);
-        cp_async_commit();
-    }
-    float          carry = 0.0f;
-    float          amax0 = 0.0f, amax1 = 0.0f;
-    SwzRot         so(lane);
-    const uint32_t prev = (lane + 31u) & 31u;
-#pragma unroll 4
-    for (uint32_t it = 0; it < 16; ++it) {
-        cp_async_wait<kRing - 1>();
-        const float4 v  = ring[(it % kRing) * 64 + lane];
-        const float  p0 = pq(v.x, r), p1 = pq(v.y, r), p2 = pq(v.z, r), p3 = pq(v.w, r);
-        const float  rot = __shfl_sync(kFull, p3, prev);
-        const float  w   = (e0 & 255u) ? (lane ? rot : carry) : 0.0f;
-        carry            = rot;
-        const float d0 = __fsub_rn(p0, w), d1 = __fsub_rn(p1, p0), d2 = __fsub_rn(p2, p1), d3 = __fsub_rn(p3, p2);
-        amax0          = fmax_nan(amax0, fabsf(d0));
-        amax1          = fmax_nan(amax1, fmax3_nan(fabsf(d1), fabsf(d2), fabsf(d3)));
-        const uint32_t m0 = static_cast<uint32_t>(fabsf(d0)), m1 = static_cast<uint32_t>(fabsf(d1));
-        const uint32_t m2 = static_cast<uint32_t>(fabsf(d2)), m3 = static_cast<uint32_t>(fabsf(d3));
-        *reinterpret_cast<uint2*>(sm + it * 64 + so.x0) =
-            make_uint2(__byte_perm(m0, m1, 0x5410) | (d0 < 0.0f ? 0x8000u : 0u), __byte_perm(m2, m3, 0x5410));
-        so.next();
-        if (signw) {
-            const uint32_t sgn = (d0 < 0.0f ? 1u : 0u) | (d1 < 0.0f ? 2u : 0u) | (d2 < 0.0f ? 4u : 0u) |
-                                 (d3 < 0.0f ? 8u : 0u);
-            uint32_t sv = sgn << ((lane & 7u) * 4);
-            sv |= __shfl_xor_sync(kFull, sv, 1);
-            sv |= __shfl_xor_sync(kFull, sv, 2);
-            sv |= __shfl_xor_sync(kFull, sv, 4);
-            if ((lane & 7u) == 0) signw[(base >> 5) + it * 4 + (lane >> 3)] = sv;
-        }
-        if (it + kRing < 16) cp_async16(rs + (it % kRing) * 1024, in + e0 + 128 * kRing, 16);
-        cp_async_commit();
         e0 += 128;
     }
     ovf |= (!(amax0 < 32768.0f) || !(amax1 < 65536.0f)) ? 1u : 0u;
@@ -900,28 +764,67 @@ __device__ void write_header(const CompressArgs& a, const EbInfo& e, uint32_t fl
 }
 
 
+// Phase C of shuffle block t: lane g holds the bit planes of group g's codes (the transposed
+// words); the shuffled image into the warp's buffer `sm`, the chunk flags as 8 ballots (=
+// bitmap words 8t..8t+7, stored) and the chunk count.  c: chunks lane + 32 i.
+__device__ __forceinline__ void flag_block(const CompressArgs& a, uint32_t t, uint32_t lane, const uint32_t (&w)[32],
+                                           uint32_t* sm, uint32_t (&bm)[8], uint32_t& cnt, uint4 (&c)[8])
+{
+    // shuffled image S[p*32 + g] = w[p] (bitshuffleAndBitflag's out, fz.cu:82)
+#pragma unroll
+    for (uint32_t p = 0; p < 32; ++p) sm[p * 32 + lane] = w[p];
+    __syncwarp();
+    // chunk c = lane + 32 i; ballot i is bitmap word 8t+i
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        c[i]  = *reinterpret_cast<const uint4*>(sm + (lane + 32 * i) * 4);
+        bm[i] = __ballot_sync(kFull, (c[i].x | c[i].y | c[i].z | c[i].w) != 0);
+        cnt += __popc(bm[i]);
+    }
+    if (lane == 0) {
+        uint4* A = reinterpret_cast<uint4*>(a.out + a.off_a) + 2 * (size_t)t;
+        A[0]     = make_uint4(bm[0], bm[1], bm[2], bm[3]);
+        A[1]     = make_uint4(bm[4], bm[5], bm[6], bm[7]);
+    }
+}
+
+// What follows the tail's codes: the zero padding of the tail code array, of the sign array
+// and of the bitmap.
+template <int ND>
+__device__ __forceinline__ void tail_pads(const CompressArgs& a, uint32_t lane, uint16_t* tc, uint32_t* signw)
+{
+    const uint32_t tail = a.n - a.nb * kBlockCodes;
+    // zero padding of the tail code array and of the sign array
+    if (tc)
+        for (uint32_t i = tail + lane; i < (uint32_t)(pad16(2 * (uint64_t)tail) / 2); i += 32) tc[i] = 0;
+    if (ND == 1 && signw) {
+        const uint32_t nsw = (uint32_t)cdiv(a.n, 32);
+        const uint32_t pw  = (uint32_t)(pad16(4 * (uint64_t)nsw) / 4);
+        for (uint32_t i = nsw + lane; i < pw; i += 32) signw[i] = 0;
+    }
+    // bitmap words of the partial block are zero (fz.cu:167), then the 16-byte pad
+    uint32_t*      A  = reinterpret_cast<uint32_t*>(a.out + a.off_a);
+    const uint32_t pa = (uint32_t)(pad16(4 * (uint64_t)a.nwords) / 4);
+    for (uint32_t i = a.nb * 8 + lane; i < pa; i += 32) A[i] = 0;
+}
+
 // Phases A-C for shuffle block t of the field: its codes into the warp's shared buffer
 // `sm` (swizzled), the bit transpose, the shuffled image back into `sm`, the chunk flags
 // as 8 ballots (= bitmap words 8t..8t+7, stored), the chunk count and the overflow bit.
 // Block t == nb (the n mod 2048 tail, never shuffled, fz.cu:173) writes its codes to the
 // sidecar and zero-fills the 16-byte pads of Sections A and C.
-// kRing > 0: the aligned 1D/2D whole-block paths take their inputs through a cp.async ring
-// of kRing group rows at `ring` (1 KiB per group row and warp).
-template <int ND, int kRing = 0>
+template <int ND>
 __device__ __forceinline__ void compute_block(const CompressArgs& a, const Geo& g, uint32_t t, float r,
                                               uint32_t lane, uint32_t* sm, uint32_t* signw,
-                                              uint32_t (&bm)[8], uint32_t& cnt, uint32_t& ovf,
-                                              float4* ring = nullptr)
+                                              uint32_t (&bm)[8], uint32_t& cnt, uint32_t& ovf)
 {
     const uint32_t base = t * kBlockCodes;
     if (t < a.nb) {
         // ---- phase A: codes of the block into shared memory (swizzled) ----
         if (ND == 1 && base + kBlockCodes <= g.nl) {
-            if constexpr (kRing > 0) block1d_ring<kRing>(a.in, base, r, lane, sm, signw, ring, ovf);
-            else block1d(a.in, base, r, lane, sm, signw, ovf);
+            block1d(a.in, base, r, lane, sm, signw, ovf);
         } else if (ND == 2 && g.al_x && base + kBlockCodes <= g.nl) {
-            if constexpr (kRing > 0) block2d_ring<kRing>(a.in, g, base, r, lane, sm, ring, ovf);
-            else block2d(a.in, g, base, r, lane, sm, ovf);
+            block2d(a.in, g, base, r, lane, sm, ovf);
         } else if (ND == 2 && g.x >= 4 && base + kBlockCodes <= g.nl) {
             block2d_u(a.in, g, base, r, lane, sm, ovf);
         } else if (ND == 3 && g.al_x && base + kBlockCodes <= g.nl) {
@@ -957,22 +860,8 @@ __device__ __forceinline__ void compute_block(const CompressArgs& a, const Geo& 
         }
         transpose32(w);
         __syncwarp();
-        // shuffled image S[p*32 + g] = w[p] (bitshuffleAndBitflag's out, fz.cu:82)
-#pragma unroll
-        for (uint32_t p = 0; p < 32; ++p) sm[p * 32 + lane] = w[p];
-        __syncwarp();
-        // ---- phase C: chunk c = lane + 32 i; ballot i is bitmap word 8t+i ----
-#pragma unroll
-        for (uint32_t i = 0; i < 8; ++i) {
-            const uint4 v = *reinterpret_cast<const uint4*>(sm + (lane + 32 * i) * 4);
-            bm[i] = __ballot_sync(kFull, (v.x | v.y | v.z | v.w) != 0);
-            cnt += __popc(bm[i]);
-        }
-        if (lane == 0) {
-            uint4* A = reinterpret_cast<uint4*>(a.out + a.off_a) + 2 * (size_t)t;
-            A[0]     = make_uint4(bm[0], bm[1], bm[2], bm[3]);
-            A[1]     = make_uint4(bm[4], bm[5], bm[6], bm[7]);
-        }
+        uint4 c[8];
+        flag_block(a, t, lane, w, sm, bm, cnt, c);
     } else if (t == a.nb && a.n > base) {
         // ---- tail block: n mod 2048 codes, never shuffled (fz.cu:173) ----
         const uint32_t tail = a.n - base;
@@ -993,18 +882,7 @@ __device__ __forceinline__ void compute_block(const CompressArgs& a, const Geo& 
                 if ((lane & 7u) == 0 && wi * 32 < a.n) signw[wi] = v;
             }
         }
-        // zero padding of the tail code array and of the sign array
-        if (tc)
-            for (uint32_t i = tail + lane; i < (uint32_t)(pad16(2 * (uint64_t)tail) / 2); i += 32) tc[i] = 0;
-        if (ND == 1 && signw) {
-            const uint32_t nsw = (uint32_t)cdiv(a.n, 32);
-            const uint32_t pw  = (uint32_t)(pad16(4 * (uint64_t)nsw) / 4);
-            for (uint32_t i = nsw + lane; i < pw; i += 32) signw[i] = 0;
-        }
-        // bitmap words of the partial block are zero (fz.cu:167), then the 16-byte pad
-        uint32_t*      A  = reinterpret_cast<uint32_t*>(a.out + a.off_a);
-        const uint32_t pa = (uint32_t)(pad16(4 * (uint64_t)a.nwords) / 4);
-        for (uint32_t i = a.nb * 8 + lane; i < pa; i += 32) A[i] = 0;
+        tail_pads<ND>(a, lane, tc, signw);
     }
     ovf = __reduce_or_sync(kFull, ovf);
 }
@@ -1162,8 +1040,8 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_compress(const Compr
 // A single field is a list of one whose job is a kernel parameter.  The stream bytes equal
 // the single-pass look-back kernel's.
 constexpr uint32_t kCompactBlocks = 32;   // shuffle blocks per compaction item
-constexpr int      kEncodeRing    = FZ_ENCODE_RING;  // group rows in flight per warp (1D/2D)
-constexpr int      kEncodeCtas    = FZ_ENCODE_CTAS;  // CTAs per SM the 1D/2D encode kernels are built for
+constexpr int      kEncodeCtas    = FZ_ENCODE_CTAS;  // CTAs per SM the encode kernels are built for
+static_assert(kItemCodes == kCompressWarps * kBlockCodes, "an encode item is a CTA's blocks");
 
 
 // ---------------------------------------------------------------- items --
@@ -1259,38 +1137,152 @@ __device__ __forceinline__ void range_items(const float* __restrict__ in, uint32
 // block's count for the compaction launch.
 constexpr uint32_t kCountPar = 1u << 31;
 
-template <int ND, int kRing>
-__device__ __forceinline__ void encode_item(const FieldJob& J, uint32_t i, float r, uint32_t par, uint32_t* sm,
-                                            float4* ring)
+// Block t's non-zero chunks (lane's: lane + 32 k) into its slot, its count into counts[] and
+// the group sums.
+__device__ __forceinline__ void emit_block(const FieldJob& J, uint32_t t, uint32_t lane, const uint4 (&c)[8],
+                                           const uint32_t (&bm)[8], uint32_t cnt, uint32_t par)
 {
-    const uint32_t      lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    uint4*         S   = J.slots + (size_t)t * kChunks;
+    const uint32_t lt  = lanemask_lt();
+    uint32_t       pre = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+        if ((bm[k] >> lane) & 1u) S[pre + __popc(bm[k] & lt)] = c[k];
+        pre += __popc(bm[k]);
+    }
+    if (lane == 0) {
+        J.counts[t] = cnt | (par ? kCountPar : 0u);
+        if (cnt) {  // into the block's group sum of each level
+            uint32_t* set = J.supers + par * J.sstride;
+            atomicAdd(set + t / kSuperBlocks, cnt);
+            atomicAdd(set + J.s2off + t / kSuper2Blocks, cnt);
+        }
+    }
+}
+
+// Block t of field J in the float path.  A call of its own: inlined, its registers would be
+// spilled around the packed path's.
+template <int ND>
+__device__ __noinline__ void float_block(const FieldJob& J, uint32_t t, float r, uint32_t par, uint32_t* sm)
+{
+    const uint32_t      lane = threadIdx.x & 31u;
     const CompressArgs& a    = J.a;
     Geo                 g;
     g.nl = a.nl, g.x = a.x, g.y = a.y, g.xy = a.xy, g.lim = a.n;
     g.dx = a.dx, g.dxy = a.dxy, g.al_x = a.al_x, g.al_xy = a.al_xy, g.al_xyx = a.al_xyx;
     uint32_t* signw = (ND == 1 && a.mode == 1) ? reinterpret_cast<uint32_t*>(a.out + a.off_sign) : nullptr;
-    const uint32_t t  = (J.ne - 1 - i) * kCompressWarps + wid;
-    uint32_t       bm[8] = {0, 0, 0, 0, 0, 0, 0, 0}, cnt = 0, ovf = 0;
-    compute_block<ND, kRing>(a, g, t, r, lane, sm, signw, bm, cnt, ovf, ring);  // warp-uniform t
+    uint32_t  bm[8] = {0, 0, 0, 0, 0, 0, 0, 0}, cnt = 0, ovf = 0;
+    compute_block<ND>(a, g, t, r, lane, sm, signw, bm, cnt, ovf);  // warp-uniform t
     if (t < a.nb) {
-        uint4*         S   = J.slots + (size_t)t * kChunks;
-        const uint32_t lt  = lanemask_lt();
-        uint32_t       pre = 0;
+        uint4 c[8];
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-            if ((bm[k] >> lane) & 1u) S[pre + __popc(bm[k] & lt)] = *reinterpret_cast<const uint4*>(sm + (lane + 32 * k) * 4);
-            pre += __popc(bm[k]);
-        }
-        if (lane == 0) {
-            J.counts[t] = cnt | (par ? kCountPar : 0u);
-            if (cnt) {  // into the block's group sum of each level
-                uint32_t* set = J.supers + par * J.sstride;
-                atomicAdd(set + t / kSuperBlocks, cnt);
-                atomicAdd(set + J.s2off + t / kSuper2Blocks, cnt);
-            }
-        }
+        for (uint32_t k = 0; k < 8; ++k) c[k] = *reinterpret_cast<const uint4*>(sm + (lane + 32 * k) * 4);
+        emit_block(J, t, lane, c, bm, cnt, par);
     }
     if (ovf && lane == 0) atomicOr(&J.ctl->flags, kCtlOverflow);
+}
+
+// The tail (n mod 2048 codes, never shuffled, fz.cu:173) from its deltas, word k at sm[k]: codes
+// into the sidecar (0 past x*y*z), signs (1D), pads.
+template <int ND>
+__device__ __noinline__ void packed_tail(const CompressArgs& a, const uint32_t* sm)
+{
+    const uint32_t lane = threadIdx.x & 31u, tb = a.nb * kBlockCodes, tail = a.n - tb;
+    uint16_t*      tc    = a.mode == 1 ? reinterpret_cast<uint16_t*>(a.out + a.off_c) : nullptr;
+    uint32_t*      signw = (ND == 1 && a.mode == 1) ? reinterpret_cast<uint32_t*>(a.out + a.off_sign) : nullptr;
+    const uint32_t in    = a.nl > tb ? a.nl - tb : 0u;  // codes inside x*y*z
+    if (tc) {
+        for (uint32_t k = lane; 2 * k < tail; k += 32) {
+            uint32_t neg, c = sign_mag2(sm[k], neg);
+            if (ND == 1) c &= (k & 1u) ? 0x7FFF7FFFu : 0x7FFFFFFFu;
+            if (2 * k < tail) tc[2 * k] = 2 * k < in ? (uint16_t)c : (uint16_t)0;
+            if (2 * k + 1 < tail) tc[2 * k + 1] = 2 * k + 1 < in ? (uint16_t)(c >> 16) : (uint16_t)0;
+        }
+    }
+    if (ND == 1 && signw) {
+        for (uint32_t i = lane; 32 * i < tail; i += 32) {
+            uint32_t v = 0;
+            for (uint32_t k = 0; k < 16; ++k) {
+                uint32_t neg;
+                sign_mag2(sm[16 * i + k], neg);
+                v |= ((neg & 1u) << (2 * k)) | ((neg >> 16) << (2 * k + 1));
+            }
+            const uint32_t live = in > 32 * i ? in - 32 * i : 0u;
+            signw[tb / 32 + i] = live >= 32 ? v : v & ((1u << live) - 1u);
+        }
+    }
+    tail_pads<ND>(a, lane, tc, signw);
+}
+
+// Block t of field J from the staged item (fz_encode.cuh), all of it inside x*y*z, or the
+// tail (t == nb).  Holds one CTA barrier: every warp has read the staged values, and the images
+// take their place.
+template <int ND, bool kRow, int kX>
+__device__ __forceinline__ void packed_block(const FieldJob& J, uint32_t t, uint32_t halo, uint32_t par, uint32_t* smem)
+{
+    const uint32_t      lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const CompressArgs& a    = J.a;
+    const uint8_t*      st   = reinterpret_cast<const uint8_t*>(smem);
+    const uint32_t      i0   = halo + (wid * 32 + lane) * 64;
+    uint32_t            w[32], bm[8], cnt = 0, slow, shigh;
+    if constexpr (ND == 1) packed_deltas1(st, i0, lane, w);
+    else packed_deltas<ND, kRow, kX>(st, i0, t * kBlockCodes + lane * 64, a.x, a.y, a.xy, a.dx, a.dxy, w);
+    __syncthreads();
+    uint32_t* sm = smem + wid * kBlockWords;
+    if (t == a.nb) {  // (warp-uniform)
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k)
+            *reinterpret_cast<uint4*>(sm + lane * 32 + 4 * k) = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+        __syncwarp();
+        packed_tail<ND>(a, sm);
+        return;
+    }
+    transpose32<true>(w);
+    sign_planes<ND == 1>(w, slow, shigh);
+    if (ND == 1 && a.mode == 1)  // the group's 64 signs, in element order
+        *reinterpret_cast<uint2*>(a.out + a.off_sign + (size_t)t * (kBlockCodes / 8) + 8 * lane) =
+            make_uint2(spread16(slow & 0xFFFFu) | (spread16(shigh & 0xFFFFu) << 1), spread16(slow >> 16) | (spread16(shigh >> 16) << 1));
+    uint4 c[8];
+    flag_block(a, t, lane, w, sm, bm, cnt, c);
+    emit_block(J, t, lane, c, bm, cnt, par);
+}
+
+// Encode item i of field J.  packed: 1 the field's range is known to fit the 16-bit path, 3 and
+// no value is negative, 2 to be found per item, 0 neither.
+template <int ND>
+__device__ __forceinline__ void encode_item(const FieldJob& J, uint32_t i, float r, uint32_t par, uint32_t packed,
+                                            uint32_t* smem)
+{
+    const uint32_t      wid  = threadIdx.x >> 5;
+    const CompressArgs& a    = J.a;
+    const uint32_t      item = J.ne - 1 - i, base = item * kItemCodes, t = item * kCompressWarps + wid;
+    StagePlan           p;
+    if (packed && base < a.nl && a.n >= 64 && stage_plan<ND>(a.x, a.xy, a.dx, a.dxy, p)) {
+        uint8_t*   stage = reinterpret_cast<uint8_t*>(smem);
+        const bool track = packed == 2;
+        float      amax  = 0.0f;
+        const bool full  = base + kItemCodes <= a.n;
+        if (packed == 3) {
+            if (full) stage_item<true, true>(a.in, a.n, base, p, r, false, stage);
+            else stage_item<true, false>(a.in, a.n, base, p, r, false, stage);
+        } else {
+            if (full) amax = stage_item<false, true>(a.in, a.n, base, p, r, track, stage);
+            else amax = stage_item<false, false>(a.in, a.n, base, p, r, track, stage);
+        }
+        if (!__syncthreads_or(track && !(amax < packed_limit<ND>()))) {
+            if ((t + 1) * kBlockCodes <= a.nl || (t == a.nb && t * kBlockCodes < a.n)) {
+                if (ND == 1) packed_block<1, false, 0>(J, t, p.halo, par, smem);
+                else if (ND == 2 && p.shift && a.al_x) packed_block<ND, false, 0>(J, t, p.halo, par, smem);
+                else if (ND == 2 && p.shift) packed_block<ND, false, 1>(J, t, p.halo, par, smem);
+                else if (a.al_x) packed_block<ND, true, 0>(J, t, p.halo, par, smem);
+                else if (a.x % 2 == 0) packed_block<ND, true, 2>(J, t, p.halo, par, smem);
+                else packed_block<ND, true, 1>(J, t, p.halo, par, smem);
+                return;
+            }
+            __syncthreads();
+        }
+    }
+    float_block<ND>(J, t, r, par, smem + wid * kBlockWords);
 }
 
 // The words the header of field J follows from, loaded by the thread that will write it as
@@ -1464,17 +1456,11 @@ __global__ void __launch_bounds__(256, FZ_RANGE_CTAS) k_range_fields(const Field
     }
 }
 
-// Ring depth (group rows in flight per warp) of the encode kernels: 1D only.  Measured on
-// GB300 (encode launch, relative eb 1e-3): 1D 2^25 elements 49.2 -> 45.3 us with 4 rows at
-// 3 CTAs/SM; 2D exafel-like 27.1 -> 29.2 us and cesm-like 16.6 -> 17.4 us, so 2D keeps its
-// one row of register lookahead at 5 CTAs/SM (the extra warps hide more than the ring).
+// Dynamic shared memory of an encode CTA: the staged item, then the warps' 4 KiB images in its
+// place.
 template <int ND>
-__host__ __device__ constexpr int encode_ring() { return ND == 1 ? kEncodeRing : 0; }
-template <int ND>
-__host__ __device__ constexpr int encode_ctas() { return ND == 3 ? 4 : (ND == 1 && kEncodeRing ? kEncodeCtas : FZ_ENCODE_CTAS_2D); }
-// Dynamic shared memory of an encode CTA: per warp the code image and the ring.
-template <int ND>
-__host__ __device__ constexpr uint32_t encode_smem() { return kCompressWarps * (kBlockWords * 4 + 1024u * encode_ring<ND>()); }
+__host__ __device__ constexpr uint32_t encode_smem() { return stage_bytes(ND == 1 ? 0u : stage_halo(kHaloRow)); }
+static_assert(encode_smem<1>() >= kCompressWarps * kBlockWords * 4, "the images fit the staging area");
 
 // Range ahead of a single-field encode launch over `total` items: the CTAs that took one
 // item fewer than the others (all CTAs when the items divide evenly; the CTAs without an
@@ -1506,20 +1492,15 @@ __device__ __forceinline__ void range_ahead(const FieldJob& J, uint32_t total)
 }
 
 template <int ND, bool kList>
-__global__ void __launch_bounds__(kCompressWarps * 32, encode_ctas<ND>())
+__global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas)
     k_encode_fields(const FieldJob* __restrict__ jobs, const Segment* __restrict__ segs, uint32_t nseg, uint32_t total,
                     const __grid_constant__ FieldJob one)
 {
     pdl_wait();
     pdl_trigger();
-    // per warp: the block's 4 KiB code image, then (1D/2D) its ring of input rows
     extern __shared__ __align__(16) uint32_t esm[];
-    constexpr int kR = encode_ring<ND>();
-    uint32_t*     smem = esm + (threadIdx.x >> 5) * kBlockWords;
-    float4*       ring = kR ? reinterpret_cast<float4*>(esm + kCompressWarps * kBlockWords) + (threadIdx.x >> 5) * kR * 64
-                            : nullptr;
     __shared__ float    s_r;
-    __shared__ uint32_t s_rf, s_par;
+    __shared__ uint32_t s_rf, s_par, s_packed;
     if (threadIdx.x == 0) s_rf = 0xFFFFFFFFu;
     for (uint32_t k = blockIdx.x; k < total; k += gridDim.x) {
         uint32_t f = 0, i = k;
@@ -1529,13 +1510,17 @@ __global__ void __launch_bounds__(kCompressWarps * 32, encode_ctas<ND>())
             // ebx2_r of the field: from its range (relative eb; complete once the range launch,
             // or the previous call's encode launch for a range ahead, has finished);
             // the call's group-sum set (the compaction launch moves the counter on)
-            s_r   = J.rel ? eb_from_range(ord2f(__ldcg(J.ctl->mm)), ord2f(__ldcg(J.ctl->mm + 1)), J.a.eb_rel).ebx2_r
-                          : J.a.ebh.ebx2_r;
+            if (J.rel) {
+                const EbInfo eb = eb_from_range(ord2f(__ldcg(J.ctl->mm)), ord2f(__ldcg(J.ctl->mm + 1)), J.a.eb_rel);
+                s_r = eb.ebx2_r, s_packed = !packed_range<ND>(eb) ? 0u : eb.vmin >= 0.0f ? 3u : 1u;
+            } else {
+                s_r = J.a.ebh.ebx2_r, s_packed = 2u;
+            }
             s_par = __ldcg(&J.ctl->epoch) & 1u;
             s_rf  = f;
         }
         __syncthreads();
-        encode_item<ND, kR>(J, i, s_r, s_par, smem, ring);
+        encode_item<ND>(J, i, s_r, s_par, s_packed, esm);
         __syncthreads();  // the blocks' shared images before the next item
         // a field without full shuffle blocks has one encode item and no compaction: the
         // header is written here (its counter stays, no group sums were used)

@@ -147,9 +147,9 @@ __device__ __forceinline__ uint32_t shr_mul(uint32_t x)
 }
 
 // One off-diagonal swap stage of width J (mask M keeps the low J bits of every 2J).
-// kMul: the shifts as multiplies -- measured on GB300 (exafel-like field): decompression
-// 21.8 -> 21.3 us, whose integer/logic pipe is its bound; the encode kernel, bound by
-// instruction issue, 27.1 -> 27.7 us, so it keeps the shifts.
+// kMul: the shifts as multiplies, where the integer/logic pipe is the bound (decompression of
+// the exafel-like field on GB300 21.8 -> 21.3 us; the staged encode); the float path of the
+// encode, bound by instruction issue, keeps the shifts (27.1 -> 27.7 us with multiplies).
 template <bool kMul, int J, uint32_t M>
 __device__ __forceinline__ void swap_stage(uint32_t (&a)[32])
 {

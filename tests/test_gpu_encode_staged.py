@@ -1,0 +1,66 @@
+"""The staged 16-bit encode (csrc/fz_encode.cuh) against the oracle, byte for byte, where it can
+go wrong: rows around its limits (64 and 4096 elements, multiples of 4, 2 and 1), items and
+tails around 16384 elements, planes shorter than an item, fields longer than their dims, values
+on rounding ties of either sign, and magnitudes around the bounds past which it hands an item
+or a field to the float path (up to deltas that overflow their codes)."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(16384, 1, 1), (16383, 1, 1), (16385, 1, 1), (40961, 1, 1), (100, 1, 1), (67, 1, 1),
+          (64, 300, 1), (65, 300, 1), (66, 299, 1), (127, 131, 1), (2049, 17, 1), (4095, 9, 1), (4096, 9, 1),
+          (4097, 9, 1), (4100, 9, 1), (4098, 33, 1), (20001, 19, 1), (63, 300, 1),
+          (64, 64, 5), (65, 7, 40), (66, 1, 300), (68, 9, 33), (64, 3, 100), (129, 127, 3), (4096, 2, 9), (4099, 3, 9),
+          (501, 37, 17), (250, 131, 9)]
+
+
+@pytest.fixture(scope="module")
+def ws(fz):
+    torch.cuda.set_device(0)
+    return fz.Workspace(1 << 20)
+
+
+def check(fz, oracle, ws, data, dims, eb, rel, mode):
+    st = fz.compress(torch.from_numpy(data).cuda(), dims, eb, rel=rel, mode=mode, ws=ws)
+    want = oracle.compress(data, dims, eb, rel=rel, mode=mode)
+    assert np.array_equal(st.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("dims", SHAPES, ids=["x".join(map(str, d)) for d in SHAPES])
+@pytest.mark.parametrize("extra", [0, 2051])
+def test_staged_streams(fz, oracle, ws, dims, extra):
+    n = dims[0] * dims[1] * dims[2] + extra
+    rng = np.random.default_rng(n)
+    half = rng.integers(-200, 201, n)  # multiples of the bound 1/2: every odd one is a rounding tie
+    for low, peak in ((-1, 1), (0, 1), (-1, 20), (-1, 75), (0, 330)):
+        data = (half * (peak * 0.5)).astype(np.float32)
+        if low == 0:
+            data = np.abs(data)
+        near = np.nextafter(data, np.float32(np.inf) * rng.choice([-1, 1], n).astype(np.float32))
+        data = np.where(rng.random(n) < 0.3, near, data).astype(np.float32)
+        if low == 0:
+            data = np.abs(data)
+        for mode in (0, 1):
+            check(fz, oracle, ws, data, dims, 0.5, False, mode)
+        # a relative bound that is (nearly) 1/2 as well
+        check(fz, oracle, ws, data, dims, 0.5 / float(data.max() - data.min()), True, 1)
+
+
+@pytest.mark.parametrize("dims", [(40000, 1, 1), (400, 101, 1), (4101, 11, 1), (70, 30, 21)],
+                         ids=["1d", "2d", "2d-wide", "3d"])
+def test_staged_bounds(fz, oracle, ws, dims):
+    """One item past the bound among others, an outlier just below and just above it, and NaN."""
+    n = dims[0] * dims[1] * dims[2]
+    rng = np.random.default_rng(1)
+    base = rng.normal(0, 30, n).astype(np.float32)
+    for peak in (4000.0, 4100.0, 8140.0, 8160.0, 16290.0, 16310.0, 32500.0, 32700.0, 66000.0, 3e9):
+        data = base.copy()
+        data[n // 2] = peak
+        check(fz, oracle, ws, data, dims, 0.5, False, 1)
+        check(fz, oracle, ws, data, dims, 0.5 / float(data.max() - data.min()), True, 1)
+        check(fz, oracle, ws, -data, dims, 0.5 / float(data.max() - data.min()), True, 1)
+    data = base.copy()
+    data[n // 3] = np.nan
+    check(fz, oracle, ws, data, dims, 0.5, False, 1)
