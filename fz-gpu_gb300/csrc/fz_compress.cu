@@ -1160,10 +1160,9 @@ __device__ __forceinline__ void emit_block(const FieldJob& J, uint32_t t, uint32
     }
 }
 
-// Block t of field J in the float path.  A call of its own: inlined, its registers would be
-// spilled around the packed path's.
+// Block t of field J in the float path.
 template <int ND>
-__device__ __noinline__ void float_block(const FieldJob& J, uint32_t t, float r, uint32_t par, uint32_t* sm)
+__device__ __forceinline__ void float_block(const FieldJob& J, uint32_t t, float r, uint32_t par, uint32_t* sm)
 {
     const uint32_t      lane = threadIdx.x & 31u;
     const CompressArgs& a    = J.a;
@@ -1217,7 +1216,7 @@ __device__ __noinline__ void packed_tail(const CompressArgs& a, const uint32_t* 
 // Block t of field J from the staged item (fz_encode.cuh), all of it inside x*y*z, or the
 // tail (t == nb).  Holds one CTA barrier: every warp has read the staged values, and the images
 // take their place.
-template <int ND, bool kRow, int kX>
+template <int ND, bool kRow, int kX, bool kNarrow>
 __device__ __forceinline__ void packed_block(const FieldJob& J, uint32_t t, uint32_t halo, uint32_t par, uint32_t* smem)
 {
     const uint32_t      lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
@@ -1226,7 +1225,7 @@ __device__ __forceinline__ void packed_block(const FieldJob& J, uint32_t t, uint
     const uint32_t      i0   = halo + (wid * 32 + lane) * 64;
     uint32_t            w[32], bm[8], cnt = 0, slow, shigh;
     if constexpr (ND == 1) packed_deltas1(st, i0, lane, w);
-    else packed_deltas<ND, kRow, kX>(st, i0, t * kBlockCodes + lane * 64, a.x, a.y, a.xy, a.dx, a.dxy, w);
+    else packed_deltas<ND, kRow, kX, kNarrow>(st, i0, t * kBlockCodes + lane * 64, a.x, a.y, a.xy, a.dx, a.dxy, w);
     __syncthreads();
     uint32_t* sm = smem + wid * kBlockWords;
     if (t == a.nb) {  // (warp-uniform)
@@ -1271,12 +1270,16 @@ __device__ __forceinline__ void encode_item(const FieldJob& J, uint32_t i, float
         }
         if (!__syncthreads_or(track && !(amax < packed_limit<ND>()))) {
             if ((t + 1) * kBlockCodes <= a.nl || (t == a.nb && t * kBlockCodes < a.n)) {
-                if (ND == 1) packed_block<1, false, 0>(J, t, p.halo, par, smem);
-                else if (ND == 2 && p.shift && a.al_x) packed_block<ND, false, 0>(J, t, p.halo, par, smem);
-                else if (ND == 2 && p.shift) packed_block<ND, false, 1>(J, t, p.halo, par, smem);
-                else if (a.al_x) packed_block<ND, true, 0>(J, t, p.halo, par, smem);
-                else if (a.x % 2 == 0) packed_block<ND, true, 2>(J, t, p.halo, par, smem);
-                else packed_block<ND, true, 1>(J, t, p.halo, par, smem);
+                const int xm = a.al_x ? 0 : a.x % 2 ? 1 : 2;  // how the row above is read
+                if (ND == 1) packed_block<1, false, 0, false>(J, t, p.halo, par, smem);
+                else if (ND == 2 && p.shift && xm == 0) packed_block<ND, false, 0, false>(J, t, p.halo, par, smem);
+                else if (ND == 2 && p.shift) packed_block<ND, false, 1, false>(J, t, p.halo, par, smem);
+                else if (a.x < 64 && xm == 0) packed_block<ND, true, 0, true>(J, t, p.halo, par, smem);
+                else if (a.x < 64 && xm == 2) packed_block<ND, true, 2, true>(J, t, p.halo, par, smem);
+                else if (a.x < 64) packed_block<ND, true, 1, true>(J, t, p.halo, par, smem);
+                else if (xm == 0) packed_block<ND, true, 0, false>(J, t, p.halo, par, smem);
+                else if (xm == 2) packed_block<ND, true, 2, false>(J, t, p.halo, par, smem);
+                else packed_block<ND, true, 1, false>(J, t, p.halo, par, smem);
                 return;
             }
             __syncthreads();

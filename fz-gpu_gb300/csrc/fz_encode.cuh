@@ -115,7 +115,7 @@ __device__ __forceinline__ bool stage_plan(uint32_t x, uint32_t xy, const FastDi
         p.halo = 0, p.shift = 0, p.tmask = 0, p.dshift = dx;
         return true;
     }
-    if (x < 64) return false;  // packed_deltas
+    if (x < 8) return false;  // packed_deltas
     if (ND == 2) {
         const bool wide = x > kHaloRow;
         p.halo  = wide ? 64u : stage_halo(x);  // wide: only the last element's difference
@@ -171,7 +171,11 @@ __device__ __forceinline__ void stage_groups(const float* __restrict__ in, uint3
             if (kAl) b[u] = __ldg(reinterpret_cast<const float4*>(bs));
             else b[u] = make_float4(__ldg(bs), __ldg(bs + 1), __ldg(bs + 2), __ldg(bs + 3));
         }
-        if (kDiff == Diff::Some) {
+        if (kDiff == Diff::Some && kAl) {
+            b[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (pos.row & p.tmask) b[u] = __ldg(reinterpret_cast<const float4*>(bs));
+            pos.next(p.shift);
+        } else if (kDiff == Diff::Some) {
             const uint32_t left = p.shift - pos.rem;  // elements of the group in this row, if < 4
             const bool     r0 = (pos.row & p.tmask) != 0, r1 = ((pos.row + 1) & p.tmask) != 0;
             b[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -278,6 +282,7 @@ __device__ __forceinline__ float stage_item(const float* __restrict__ in, uint32
         if (p.shift % 4 == 0) return stage_segment<Diff::All, true, kPos, kFull>(in, n, base, p, r, track, st);
         return stage_segment<Diff::All, false, kPos, kFull>(in, n, base, p, r, track, st);
     }
+    if (p.shift % 4 == 0) return stage_segment<Diff::Some, true, kPos, kFull>(in, n, base, p, r, track, st);
     return stage_segment<Diff::Some, false, kPos, kFull>(in, n, base, p, r, track, st);
 }
 
@@ -308,18 +313,19 @@ __device__ __forceinline__ void packed_deltas1(const uint8_t* st, uint32_t i0, u
     }
 }
 
-// 2D and 3D; x >= 64, so that a lane's 64 elements end a row at most once.  kRow: subtract the
-// row above (2D with the row staged, 3D).  kX: x % 4 where the row above is read (0, 2, or 1
-// for any odd x).  The end of a row inside a group of 4 is behind a test of a warp-wide mask;
-// which elements start a tile row repeats every 16 (8) elements and is kept as masks.
-template <int ND, bool kRow, int kX>
+// 2D and 3D.  kRow: subtract the row above (2D with the row staged, 3D).  kX: x % 4 where the row
+// above is read (0, 2, or 1 for any odd x).  Rows of 64 elements and more end at most once in
+// a lane's 64: that end, inside a group of 4, is behind a test of a warp-wide mask, and which
+// elements start a tile row -- every 16th (8th) -- is kept as masks.  kNarrow (8 <= x < 64):
+// both are found for each group.
+template <int ND, bool kRow, int kX, bool kNarrow>
 __device__ __forceinline__ void packed_deltas(const uint8_t* st, uint32_t i0, uint32_t e0, uint32_t x, uint32_t y,
                                               uint32_t xy, const FastDiv& dx, const FastDiv& dxy, uint32_t (&w)[32])
 {
     constexpr uint32_t tw = ND == 2 ? 15u : 7u;  // tile width - 1
     constexpr int      kPer = (tw + 1) / 2;      // words of its period
     const uint8_t*     pc = st + (i0 >> 6) * kStageSlot;  // i0 % 64 == 0
-    uint32_t           rw, col;  // row (3D: of the plane) and column of e0
+    uint32_t           rw, col;  // row (3D: of the plane) and column of e0 (kNarrow: of the group)
     if (ND == 2) {
         rw = fdiv(e0, dx), col = e0 - rw * x;
     } else {
@@ -327,10 +333,10 @@ __device__ __forceinline__ void packed_deltas(const uint8_t* st, uint32_t i0, ui
         rw = fdiv(rem, dx), col = rem - rw * x;
     }
     const uint32_t q   = x - col;  // elements left in the row; the next row's first is element q (if < 64)
-    const uint32_t rwn = ND == 3 && rw + 1 == y ? 0u : rw + 1;
+    uint32_t       rwn = ND == 3 && rw + 1 == y ? 0u : rw + 1;
     uint32_t       my  = (rw & tw) ? kFull : 0u;  // the row above lies in the tile
-    const uint32_t myn = (rwn & tw) ? kFull : 0u;
-    const uint32_t wu  = __reduce_or_sync(kFull, q < 64 ? 1u << (q >> 2) : 0u);  // groups with a row's first element
+    uint32_t       myn = (rwn & tw) ? kFull : 0u;
+    const uint32_t wu  = kNarrow ? 0u : __reduce_or_sync(kFull, q < 64 ? 1u << (q >> 2) : 0u);  // groups with a row's first element
     // halves of the words w, w + kPer, ... that start a tile row (kX == 0: low halves only)
     uint32_t sm[kPer];
     auto starts = [&](uint32_t k) {  // element k of the period starts one
@@ -358,7 +364,22 @@ __device__ __forceinline__ void packed_deltas(const uint8_t* st, uint32_t i0, ui
     for (int j = 0; j < 16; ++j) {
         const uint2 c   = *reinterpret_cast<const uint2*>(pc + 8 * j);
         uint32_t    t01 = c.x, t23 = c.y, m0 = my, m1 = my, s0 = sm[2 * j % kPer], s1 = sm[(2 * j + 1) % kPer];
-        if (wu & (1u << j)) {  // (warp-uniform)
+        if (kNarrow) {
+            const uint32_t k = (0u - col) & tw;  // element k starts a tile row (if < 4)
+            s0 = k == 0 ? 0xFFFFu : k == 1 ? 0xFFFF0000u : 0u, s1 = k == 2 ? 0xFFFFu : k == 3 ? 0xFFFF0000u : 0u;
+            col += 4;
+            if (col >= x) {  // the group ends its row; its last col elements are in the next
+                col -= x;
+                uint32_t o0, o1, f0, f1;  // elements of the old row, and those and the new row's first
+                low_halves(4 - col, o0, o1);
+                low_halves(col ? 5 - col : 4u, f0, f1);
+                m0 = pick(o0, my, myn), m1 = pick(o1, my, myn), my = myn;
+                s0 = (s0 & o0) | (f0 & ~o0), s1 = (s1 & o1) | (f1 & ~o1);
+                ++rwn;
+                if (ND == 3 && rwn == y) rwn = 0;
+                myn = (rwn & tw) ? kFull : 0u;
+            }
+        } else if (wu & (1u << j)) {  // (warp-uniform)
             if ((q >> 2) == (uint32_t)j) {
                 uint32_t o0, o1;  // elements of the old row
                 low_halves(q & 3u, o0, o1);

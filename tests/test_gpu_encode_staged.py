@@ -1,5 +1,5 @@
 """The staged 16-bit encode (csrc/fz_encode.cuh) against the oracle, byte for byte, where it can
-go wrong: rows around its limits (64 and 4096 elements, multiples of 4, 2 and 1), items and
+go wrong: rows around its limits (8, 64 and 4096 elements, multiples of 4, 2 and 1), items and
 tails around 16384 elements, planes shorter than an item, fields longer than their dims, values
 on rounding ties of either sign, and magnitudes around the bounds past which it hands an item
 or a field to the float path (up to deltas that overflow their codes)."""
@@ -13,7 +13,9 @@ SHAPES = [(16384, 1, 1), (16383, 1, 1), (16385, 1, 1), (40961, 1, 1), (100, 1, 1
           (64, 300, 1), (65, 300, 1), (66, 299, 1), (127, 131, 1), (2049, 17, 1), (4095, 9, 1), (4096, 9, 1),
           (4097, 9, 1), (4100, 9, 1), (4098, 33, 1), (20001, 19, 1), (63, 300, 1),
           (64, 64, 5), (65, 7, 40), (66, 1, 300), (68, 9, 33), (64, 3, 100), (129, 127, 3), (4096, 2, 9), (4099, 3, 9),
-          (501, 37, 17), (250, 131, 9)]
+          (501, 37, 17), (250, 131, 9), (8, 2100, 1), (9, 2000, 1), (10, 1900, 1), (12, 1500, 1), (17, 1001, 1),
+          (33, 500, 1), (62, 290, 1), (8, 8, 60), (9, 5, 400), (13, 1, 1500), (31, 43, 13), (48, 20, 30), (62, 70, 5),
+          (7, 900, 1), (6, 50, 70)]
 
 
 @pytest.fixture(scope="module")
