@@ -444,16 +444,8 @@ def check_recon(X, Y, headers):
 
 
 def decompress_kernel(dims):
-    """The fused decompression kernel the library runs for these dims (the name ncu shows):
-    2D rows a multiple of 16 elements take k_decompress2d_x16 when its grid of 960-column x
-    16-row windows fits one resident wave (3 CTAs per SM)."""
-    import torch
-    nd = 3 if dims[2] > 1 else (2 if dims[1] > 1 else 1)
-    if nd == 2 and dims[0] % 16 == 0:
-        ctas = -(-dims[0] // 960) * -(-dims[1] // 16)
-        if ctas <= 3 * torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count:
-            return "k_decompress2d_x16"
-    return f"k_decompress{nd}d"
+    """The fused decompression kernel the library runs for these dims (the name ncu shows)."""
+    return f"k_decompress{3 if dims[2] > 1 else (2 if dims[1] > 1 else 1)}d"
 
 
 def kernel_table(kern, n, stream_b, dims, hbm):

@@ -4,9 +4,9 @@
 //              stream straight into the field: each CTA decodes the 64-code groups its
 //              rows (or 256-element blocks) need -- rank of every flagged chunk from the
 //              bitmap and the block offset table, inverse 32x32 bit transposes -- then
-//              runs the per-tile inclusive prefix sums in 32-bit integers (1D 256, 2D
-//              16x16, 3D 8x8x8 -- the tiling of x_lorenzo_{1d,2d,3d},
-//              lorenzo_var.cuh:297-518) and writes (float)p * ebx2.
+//              runs the per-tile inclusive prefix sums (1D 256, 2D 16x16, 3D 8x8x8 -- the
+//              tiling of x_lorenzo_{1d,2d,3d}, lorenzo_var.cuh:297-518) in 32-bit integers
+//              (1D) or in floats that hold them exactly, and writes p * ebx2.
 //   k_offsets  block offset table from the bitmap (COMPAT streams, which carry none).
 //   k_recon{1,2,3}d  inverse Lorenzo of a code array (the stage-level API,
 //              fz_lorenzo_reconstruct).
@@ -145,315 +145,366 @@ __device__ __forceinline__ void sm_decode2(uint32_t w, uint32_t& d0, uint32_t& d
     d1 = ((__byte_perm(w, 0u, 0x4432) & 0x7FFFu) ^ m1) - m1;
 }
 
-// Decodes the 64 codes of group g (codes g*64 .. g*64+63) into 32 words w[j] =
-// code[2j] | code[2j+1] << 16.  Group gg of block b is word r4 = gg % 4 of the 32
-// chunks (p, k = gg / 4): its rank among the flagged chunks follows from the block's
-// bitmap and its offset boff[b].  Groups past the last full block read the sidecar.
-__device__ __forceinline__ void decode_group(const DecodeArgs& a, uint32_t g, uint32_t (&w)[32])
+// *p where cond is not 0, 0 elsewhere: a predicated load (the compiler makes a branch of the
+// conditional expression).
+__device__ __forceinline__ uint32_t ldg_if(const uint32_t* p, uint32_t cond)
 {
-    const uint32_t b = g >> 5;
-    if (b < a.nb) {
-        const uint32_t gg = g & 31u, k = gg >> 2, r4 = gg & 3u;
-        const uint4*   A4 = reinterpret_cast<const uint4*>(a.st + a.off_a) + 2 * (size_t)b;
-        const uint4    b0 = __ldg(A4), b1 = __ldg(A4 + 1);
-        const uint32_t bm[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-        const uint32_t base  = __ldg(a.boff + b);
-        const uint32_t* W4   = reinterpret_cast<const uint32_t*>(a.st + a.off_b) + r4;
-        // chunk c = 8p + k sits in bitmap word p/4 at bit 8(p%4) + k
-        uint32_t lowm[4], bit[4];
+    uint32_t v;
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; mov.u32 %0, 0; @q ld.global.nc.u32 %0, [%1]; }"
+                 : "=r"(v)
+                 : "l"(p), "r"(cond));
+    return v;
+}
+
+// Bit planes of 32 words of two sign-magnitude codes (plane p of the low codes in w[p], of the
+// high ones in w[16 + p]) to the planes of their deltas plus 0x8000: where the sign is set the
+// magnitude is negated with a rippling carry, then the top bit inverted -- two three-input
+// operations a plane, instead of several per code after the transpose.  (A set sign on a zero
+// magnitude is zero, as in sm_decode.)
+__device__ __forceinline__ void delta_planes(uint32_t (&w)[32])
+{
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            bit[q]  = 1u << (8 * q + k);
-            lowm[q] = bit[q] - 1u;
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t s = w[16 * h + 15];
+        uint32_t       c = s;
+#pragma unroll
+        for (int p = 0; p < 15; ++p) {
+            const uint32_t b = w[16 * h + p];
+            w[16 * h + p]    = b ^ s ^ c;
+            c                = (b ^ s) & c;
         }
-        uint32_t       pw  = base;
-        const uint32_t end = __ldg(a.boff + b + 1);
-        // the table agrees with the bitmap and the block's chunks lie inside the stream:
-        // then every rank below is < nnz; otherwise nothing is read
-        const bool bad = end - base != (uint32_t)(__popc(b0.x) + __popc(b0.y) + __popc(b0.z) + __popc(b0.w) +
-                                                  __popc(b1.x) + __popc(b1.y) + __popc(b1.z) + __popc(b1.w)) ||
-                         end < base || end > a.nnz;
-        const uint32_t live = bad ? 0u : kFull;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t bmi = bm[i] & live;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int      p    = 4 * i + q;
-                const uint32_t rank = pw + __popc(bmi & lowm[q]);
-                w[p]                = (bmi & bit[q]) ? __ldg(W4 + 4 * (size_t)rank) : 0u;
-            }
-            pw += __popc(bmi);
-        }
-        if (bad) atomicOr(a.status, kStatusCorrupt);
-        transpose32<true>(w);  // w[p] = S[p*32 + gg]  ->  w[j] = W[gg*32 + j]
-    } else {
-        const uint16_t* tc  = a.mode == 1 ? reinterpret_cast<const uint16_t*>(a.st + a.off_c) : nullptr;
-        const uint32_t  e0  = g * 64;
-        const uint32_t  tb  = a.nb * kBlockCodes;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const uint32_t e  = e0 + 2 * j;
-            const uint32_t lo = (tc && e < a.n) ? tc[e - tb] : 0u;
-            const uint32_t hi = (tc && e + 1 < a.n) ? tc[e + 1 - tb] : 0u;
-            w[j] = lo | (hi << 16);
-        }
+        w[16 * h + 15] = ~(s ^ c);
     }
 }
 
-// Decoded row buffers (fused 2D/3D paths): a row of the field's window is held as 64-code
-// slots (one decode group each) of eight 16-byte chunks, in one of two layouts:
-//   padded (2D): code e at word (e / 64) * kSlotWords + (e % 64) / 2.  The 16-byte pad
-//     per slot puts neighbouring slots 4 banks apart, so the 16-byte stores of 8 threads
-//     writing chunk tt of consecutive groups hit distinct banks, and a read address is a
-//     shift, a mask and a multiply-add.
-//   swizzled (3D, whose kernel runs at its register limit): 32 words per slot, chunk c of
-//     slot G at chunk position c ^ (G & 7).
+// Two sign-magnitude codes of a word as deltas plus 0x8000 (the few codes outside the shuffled
+// blocks).
+__device__ __forceinline__ uint32_t delta_word(uint32_t w)
+{
+    return ((sm_decode(w & 0xFFFFu) + 0x8000u) & 0xFFFFu) | ((sm_decode(w >> 16) + 0x8000u) << 16);
+}
+
+// A lane's group gg of block b is word r4 = gg % 4 of the 32 chunks (p, k = gg / 4): the ranks of
+// those among the flagged chunks follow from the block's bitmap and its offset boff[b].  bm
+// holds the bitmap (chunk (p, k) at bit 8 (p % 4) + k of word p / 4), all zero when the offset
+// table disagrees with it or the block's chunks lie outside the stream (nothing is read then);
+// W4 the word r4 of the block's first chunk.
+struct GroupBits {
+    uint32_t        bm[8], k;
+    const uint32_t* W4;
+};
+__device__ __forceinline__ GroupBits group_bits(const DecodeArgs& a, uint32_t g)
+{
+    GroupBits      G;
+    const uint32_t b = g >> 5;
+    const uint4*   A4 = reinterpret_cast<const uint4*>(a.st + a.off_a) + 2 * (size_t)b;
+    const uint4    b0 = __ldg(A4), b1 = __ldg(A4 + 1);
+    const uint32_t base = __ldg(a.boff + b), end = __ldg(a.boff + b + 1);
+    G.k  = (g & 31u) >> 2;
+    G.W4 = reinterpret_cast<const uint32_t*>(a.st + a.off_b) + (g & 3u) + 4 * (size_t)base;
+    // then every rank below is < nnz
+    const bool bad = end - base != (uint32_t)(__popc(b0.x) + __popc(b0.y) + __popc(b0.z) + __popc(b0.w) +
+                                              __popc(b1.x) + __popc(b1.y) + __popc(b1.z) + __popc(b1.w)) ||
+                     end < base || end > a.nnz;
+    const uint32_t live = bad ? 0u : kFull;
+    G.bm[0] = b0.x & live, G.bm[1] = b0.y & live, G.bm[2] = b0.z & live, G.bm[3] = b0.w & live;
+    G.bm[4] = b1.x & live, G.bm[5] = b1.y & live, G.bm[6] = b1.z & live, G.bm[7] = b1.w & live;
+    if (bad) atomicOr(a.status, kStatusCorrupt);
+    return G;
+}
+// Planes 4 i + q, q in [q0, q1), into w[4 i + q]; W4 moves past the word's chunks.
+template <int i, int q0, int q1>
+__device__ __forceinline__ void gather_planes(GroupBits& G, uint32_t* w)
+{
+#pragma unroll
+    for (int q = q0; q < q1; ++q) {
+        const uint32_t bit = 1u << (8 * q + G.k);
+        w[q] = ldg_if(G.W4 + 4 * __popc(G.bm[i] & (bit - 1u)), G.bm[i] & bit);
+    }
+    G.W4 += 4 * __popc(G.bm[i]);
+}
+
+// Plane 4 i + 3 alone.
+template <int i>
+__device__ __forceinline__ void gather_sign(GroupBits& G, uint32_t& w)
+{
+    const uint32_t bit = 1u << (24 + G.k);
+    w = ldg_if(G.W4 + 4 * __popc(G.bm[i] & (bit - 1u)), G.bm[i] & bit);
+    G.W4 += 4 * __popc(G.bm[i]);
+}
+
+// The 64 codes of group g (codes g*64 .. g*64+63) as 32 words w[j] = code[2j] | code[2j+1] << 16.
+// Groups past the last full block read the sidecar.
+__device__ __forceinline__ void tail_group(const DecodeArgs& a, uint32_t g, uint32_t (&w)[32])
+{
+    const uint16_t* tc  = a.mode == 1 ? reinterpret_cast<const uint16_t*>(a.st + a.off_c) : nullptr;
+    const uint32_t  e0  = g * 64;
+    const uint32_t  tb  = a.nb * kBlockCodes;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        const uint32_t e  = e0 + 2 * j;
+        const uint32_t lo = (tc && e < a.n) ? tc[e - tb] : 0u;
+        const uint32_t hi = (tc && e + 1 < a.n) ? tc[e + 1 - tb] : 0u;
+        w[j] = lo | (hi << 16);
+    }
+}
+__device__ __forceinline__ void gather_group(GroupBits& G, uint32_t (&w)[32])
+{
+    gather_planes<0, 0, 4>(G, w);
+    gather_planes<1, 0, 4>(G, w + 4);
+    gather_planes<2, 0, 4>(G, w + 8);
+    gather_planes<3, 0, 4>(G, w + 12);
+    gather_planes<4, 0, 4>(G, w + 16);
+    gather_planes<5, 0, 4>(G, w + 20);
+    gather_planes<6, 0, 4>(G, w + 24);
+    gather_planes<7, 0, 4>(G, w + 28);
+}
+__device__ __forceinline__ void decode_group(const DecodeArgs& a, uint32_t g, uint32_t (&w)[32])
+{
+    if ((g >> 5) < a.nb) {
+        GroupBits G = group_bits(a, g);
+        gather_group(G, w);
+        transpose32<true>(w);  // w[p] = S[p*32 + gg]  ->  w[j] = W[gg*32 + j]
+    } else {
+        tail_group(a, g, w);
+    }
+}
+
+// Both deltas of byte c of the low and of the high word, sign-extended, plus 0x8000.
+template <int c>
+__device__ __forceinline__ uint32_t delta_bytes(uint32_t lo, uint32_t hi)
+{
+    uint32_t r;  // bytes c, its sign, 4 + c, its sign (prmt mode 8 + byte)
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(lo), "r"(hi), "n"(0xC480 + 0x1111 * c));
+    return r ^ 0x80008000u;
+}
+
+// The 64 deltas of group g plus 0x8000, two per word as decode_group's codes; all lanes of the
+// warp call it, those without a group (valid false) get some values.  Where no lane of the warp
+// has a magnitude of 2^7 or more -- most warps of a compressible stream: only tile corners
+// hold values instead of differences -- planes 7..14 of either half are neither fetched nor
+// transposed: 16 planes as bytes, widened at the end.
+__device__ __forceinline__ void decode_deltas(const DecodeArgs& a, uint32_t g, bool valid, uint32_t (&w)[32])
+{
+    const bool in_block = valid && (g >> 5) < a.nb;
+    GroupBits  G;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) G.bm[i] = 0;
+    G.k = 0, G.W4 = nullptr;
+    if (in_block) G = group_bits(a, g);
+    const uint32_t high = ((G.bm[1] & 0xFF000000u) | G.bm[2] | (G.bm[3] & 0x00FFFFFFu) | (G.bm[5] & 0xFF000000u) | G.bm[6] |
+                           (G.bm[7] & 0x00FFFFFFu)) & (0x01010101u << G.k);
+    if (!__any_sync(kFull, high != 0 || (valid && !in_block))) {
+        uint32_t t[2][8], s[2];
+        gather_planes<0, 0, 4>(G, t[0]);
+        gather_planes<1, 0, 3>(G, t[0] + 4);
+        gather_planes<2, 0, 0>(G, nullptr);
+        gather_sign<3>(G, s[0]);
+        gather_planes<4, 0, 4>(G, t[1]);
+        gather_planes<5, 0, 3>(G, t[1] + 4);
+        gather_planes<6, 0, 0>(G, nullptr);
+        gather_sign<7>(G, s[1]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // as delta_planes, the sign plane kept
+            uint32_t c = s[h];
+#pragma unroll
+            for (int p = 0; p < 7; ++p) {
+                const uint32_t b = t[h][p];
+                t[h][p]          = b ^ s[h] ^ c;
+                c                = (b ^ s[h]) & c;
+            }
+            t[h][7] = s[h] ^ c;
+            transpose8(t[h]);  // byte c of t[h][i]: the delta of pair 8 c + i
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            w[i]      = delta_bytes<0>(t[0][i], t[1][i]);
+            w[8 + i]  = delta_bytes<1>(t[0][i], t[1][i]);
+            w[16 + i] = delta_bytes<2>(t[0][i], t[1][i]);
+            w[24 + i] = delta_bytes<3>(t[0][i], t[1][i]);
+        }
+        return;
+    }
+    if (in_block) {
+        gather_group(G, w);
+        delta_planes(w);
+        transpose32<true>(w);
+    } else if (valid) {
+        tail_group(a, g, w);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) w[j] = delta_word(w[j]);
+    }
+}
+
+// Decoded row buffers (fused 2D/3D paths): a row of the field's window is held as 64-code slots
+// (one decode group each) of 36 words: code e at word (e / 64) * 36 + (e % 64) / 2.  The
+// 16-byte pad per slot puts neighbouring slots 4 banks apart, so the 16-byte stores of 8
+// threads writing chunk tt of consecutive groups hit distinct banks; it repeats the next
+// slot's first two words, so that 5 codes from anywhere are three words in a row.
 constexpr uint32_t kSlotWords = 36;
 
-// word of chunk c of slot G
-template <bool kPad>
-__device__ __forceinline__ uint32_t rb_chunk(uint32_t G, uint32_t c)
-{
-    return kPad ? G * kSlotWords + 4 * c : (G * 8 + (c ^ (G & 7u))) << 2;
-}
-// word holding code e
-template <bool kPad>
-__device__ __forceinline__ uint32_t rb_word(uint32_t e)
-{
-    return kPad ? (e >> 6) * kSlotWords + ((e & 63u) >> 1) : rb_chunk<false>(e >> 6, (e >> 3) & 7u) + ((e >> 1) & 3u);
-}
+// word holding code e: e / 2 + 4 (e / 64)
+__device__ __forceinline__ uint32_t rb_word(uint32_t e) { return (e >> 1) + 4 * (e >> 6); }
 
-template <bool kPad>
+// Group j's deltas into slot j; kPads: the first two words into the pad of the slot before too.
+template <bool kPads>
 __device__ __forceinline__ void rb_put_group(uint32_t* rb, uint32_t j, const uint32_t (&w)[32])
 {
 #pragma unroll
     for (uint32_t tt = 0; tt < 8; ++tt)
-        *reinterpret_cast<uint4*>(rb + rb_chunk<kPad>(j, tt)) =
+        *reinterpret_cast<uint4*>(rb + j * kSlotWords + 4 * tt) =
             make_uint4(w[4 * tt], w[4 * tt + 1], w[4 * tt + 2], w[4 * tt + 3]);
+    if (kPads && j) *reinterpret_cast<uint2*>(rb + j * kSlotWords - 4) = make_uint2(w[0], w[1]);
 }
 
-// Integer deltas of codes i..i+3 of a row buffer.  i % 4 is the same for every thread of
-// a row, so the branch is uniform.
-template <bool kPad>
-__device__ __forceinline__ void rb_read4(const uint32_t* rb, uint32_t i, uint32_t (&d)[4])
+// The deltas (plus 0x8000) of codes i..i+3 of a row buffer as two words of two.  kAl: i % 4 == 0.
+template <bool kAl>
+__device__ __forceinline__ void rb_read4(const uint32_t* rb, uint32_t i, uint32_t& x01, uint32_t& x23)
 {
-    if ((i & 3u) == 0) {
-        const uint2 v = *reinterpret_cast<const uint2*>(rb + rb_word<kPad>(i));
-        sm_decode2(v.x, d[0], d[1]);
-        sm_decode2(v.y, d[2], d[3]);
+    const uint32_t* p = rb + rb_word(i);
+    if (kAl) {
+        const uint2 v = *reinterpret_cast<const uint2*>(p);
+        x01 = v.x, x23 = v.y;
     } else {
-#pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) {
-            const uint32_t e  = i + k;
-            const uint32_t wv = rb[rb_word<kPad>(e)];
-            d[k]              = sm_decode((e & 1u) ? wv >> 16 : wv & 0xFFFFu);
+        const uint32_t u = p[0], v = p[1], w = p[2], sel = (i & 1u) ? 0x5432u : 0x3210u;
+        x01 = __byte_perm(u, v, sel), x23 = __byte_perm(v, w, sel);
+    }
+}
+
+// Prefix sums in float, two values per instruction (add/mul.f32x2).  Every partial sum is an
+// integer of at most 512 deltas below 2^15 (an 8x8x8 tile; 256 in 2D), so below 2^24 and exact:
+// the sums equal the 32-bit integer ones and their product with ebx2 is bit-identical.
+struct Pair {
+    float x, y;
+};
+__device__ __forceinline__ Pair add2(Pair a, Pair b)
+{
+    Pair r;
+    asm("{ .reg .b64 s, t; mov.b64 s, {%2, %3}; mov.b64 t, {%4, %5}; add.rn.f32x2 s, s, t; mov.b64 {%0, %1}, s; }"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ Pair mul2(Pair a, float b)
+{
+    Pair r;
+    asm("{ .reg .b64 s, t; mov.b64 s, {%2, %3}; mov.b64 t, {%4, %4}; mul.rn.f32x2 s, s, t; mov.b64 {%0, %1}, s; }"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b));
+    return r;
+}
+// Both deltas of a word of two plus 0x8000: each half under the exponent of 2^23, less 2^23 + 2^15.
+__device__ __forceinline__ Pair delta2(uint32_t x)
+{
+    const Pair f{__uint_as_float(__byte_perm(x, 0x4B000000u, 0x7410)), __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7432))};
+    return add2(f, Pair{-8421376.0f, -8421376.0f});
+}
+
+// Stores min(live, 4) reconstructed values at out (none for live <= 0).  kAl: all 4, 16-byte
+// aligned.  (Rows that start anywhere: gathering the aligned groups of 4 from neighbouring threads
+// by shuffle took more instructions than its wider stores saved, 501x500x100 on GB300 46.6 ->
+// 49.1 us.)
+template <bool kAl>
+__device__ __forceinline__ void store_row(float* out, int32_t live, Pair a, Pair b, float ebx2)
+{
+    const Pair f = mul2(a, ebx2), g = mul2(b, ebx2);
+    if (kAl) {
+        if (live > 0) *reinterpret_cast<float4*>(out) = make_float4(f.x, f.y, g.x, g.y);
+    } else if (live >= 4) {
+        if ((reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+            *reinterpret_cast<float4*>(out) = make_float4(f.x, f.y, g.x, g.y);
+        } else {
+            out[0] = f.x, out[1] = f.y, out[2] = g.x, out[3] = g.y;
         }
+    } else if (live > 0) {
+        out[0] = f.x;
+        if (live > 1) out[1] = f.y;
+        if (live > 2) out[2] = g.x;
     }
 }
 
-// Stores min(live, 4) reconstructed values at element lin (16-byte store when aligned).
-__device__ __forceinline__ void store4(float* out, uint32_t lin, uint32_t live, const uint32_t (&acc)[4], float ebx2)
+// A thread's 4 deltas of a row to the sums along x up to its 4 columns: serially, then over the
+// threads of the tile row (kQuads threads of 4 columns, q this one's place).
+template <int kQuads>
+__device__ __forceinline__ void sums_x(uint32_t x01, uint32_t x23, uint32_t q, Pair& a, Pair& b)
 {
-    const float f0 = (float)(int32_t)acc[0] * ebx2, f1 = (float)(int32_t)acc[1] * ebx2;
-    const float f2 = (float)(int32_t)acc[2] * ebx2, f3 = (float)(int32_t)acc[3] * ebx2;
-    if (live >= 4 && (lin & 3u) == 0) {
-        *reinterpret_cast<float4*>(out + lin) = make_float4(f0, f1, f2, f3);
+    a = delta2(x01), b = delta2(x23);
+    a.y += a.x, b.x += a.y, b.y += b.x;
+    float v = b.y, u = __shfl_up_sync(kFull, v, 1);
+    if (kQuads == 2) {
+        u = (q & 1u) ? u : 0.0f;
     } else {
-        out[lin] = f0;
-        if (live > 1) out[lin + 1] = f1;
-        if (live > 2) out[lin + 2] = f2;
-        if (live > 3) out[lin + 3] = f3;
+        if (q >= 1) v += u;
+        u = __shfl_up_sync(kFull, v, 2);
+        if (q >= 2) v += u;
+        u = v - b.y;
     }
+    a = add2(a, Pair{u, u}), b = add2(b, Pair{u, u});
 }
 
 // ------------------------------------------------------ fused 2D decode --
 // A CTA owns a 16-row tile band and a 960-column window (60 tile columns); the flat
 // block index runs over windows fastest.  Phase 1: thread (row rr, j) decodes group
 // glo(rr) + j of that row's span into the row buffer.  Phase 2: thread t owns columns
-// 4t..4t+3; prefix along x (serial + quad shuffles), running sum along y, (float)p *
-// ebx2, coalesced stores.  Traffic: the chunks once (plus the at most two groups a row
-// shares with the next window) and the output once.
-constexpr uint32_t kW2 = 960;
+// 4t..4t+3; prefix along x (serial + quad shuffles), running sum along y, times ebx2,
+// coalesced stores.  Traffic: the chunks once (plus the at most two groups a row shares
+// with the next window) and the output once.
+//
+// Bound by instruction issue (70%), then by the tail of a last wave.  GB300, event-timed, with
+// the signs undone in the bit planes, planes 7..14 left out where a warp has none, and the sums
+// in float pairs, against a sign per code and integer sums: 39200x388 20.7 -> 18.5 us,
+// 8192x8192 69.7 -> 57.5, 3601x1801 16.9 -> 14.6; 3600x1800 12.6 as with the separate kernel for
+// x % 16 == 0 (12.3-13.0) that it replaces.  256 threads, 4 CTAs an SM (64 registers): 5 CTAs of
+// 48 registers spill (3600x1800 13.5 us, 39200x388 18.8, 8192x8192 56.1); 128 threads with
+// 448-column windows lose as much to the groups shared between windows (14.1, 19.0, 59.5).
+constexpr uint32_t kT2 = 256;            // threads
+constexpr uint32_t kW2 = 4 * kT2 - 64;   // columns of a window: their codes touch at most kT2 / 16 groups a row
 
-// kAl: x % 4 == 0.  Windows start at multiples of 960 columns, so every row's window then
+// kAl: x % 4 == 0.  Windows start at multiples of kW2 columns, so every row's window then
 // starts on a 4-code boundary: a thread's 4 codes are one 8-byte pair of row-buffer words,
 // its 4 outputs one 16-byte store (c1 - c0 is a multiple of 4, so a live thread has all
 // 4 columns), and nothing about alignment or width is decided per row.
 template <bool kAl>
-__global__ void __launch_bounds__(256, 5) k_decompress2d(const DecodeArgs a, uint32_t nwin)
+__global__ void __launch_bounds__(kT2, 4) k_decompress2d(const DecodeArgs a, uint32_t nwin)
 {
     pdl_wait();
     pdl_trigger();
-    __shared__ __align__(16) uint32_t rows[16][16 * kSlotWords];  // 16 rows x 16 slots of 64 codes
+    constexpr uint32_t kG = kT2 / 16;  // groups per row
+    __shared__ __align__(16) uint32_t rows[16][kG * kSlotWords];
     const uint32_t tid = threadIdx.x;
     const uint32_t bx = blockIdx.x % nwin, by = blockIdx.x / nwin;
     const uint32_t c0 = bx * kW2, c1 = min(c0 + kW2, a.x);
     const uint32_t r0 = by * 16;
     {
-        const uint32_t rr = tid >> 4, j = tid & 15u, row = r0 + rr;
-        if (row < a.y) {
-            const uint32_t lin0 = row * a.x + c0, lin1 = row * a.x + c1;
-            const uint32_t g = (lin0 >> 6) + j;
-            if (g <= ((lin1 - 1) >> 6)) {
-                uint32_t w[32];
-                decode_group(a, g, w);
-                rb_put_group<true>(rows[rr], j, w);
-            }
-        }
+        const uint32_t rr = tid / kG, j = tid % kG, row = r0 + rr;
+        const uint32_t lin0 = row * a.x + c0, g = (lin0 >> 6) + j;
+        const bool     valid = row < a.y && g <= ((lin0 + (c1 - c0) - 1) >> 6);
+        uint32_t       w[32];
+        decode_deltas(a, g, valid, w);
+        if (valid) rb_put_group<!kAl>(rows[rr], j, w);
     }
     __syncthreads();
     const uint32_t col  = c0 + 4 * tid;
     const bool     live = col < c1;
     const uint32_t q    = tid & 3u;
-    uint32_t       acc[4] = {0, 0, 0, 0};
-    if (kAl) {
-        const uint32_t nrows = min(16u, a.y - r0);
-        uint32_t       lin0  = r0 * a.x + c0;  // first code of the window in row r0 + rr
-        // threads past the window's end read the row's first word (in bounds; their values
-        // only reach higher quad positions, which are past the end too, and are not stored)
-        const uint32_t t4 = live ? 4 * tid : 0u;
-#pragma unroll 4
-        for (uint32_t rr = 0; rr < 16; ++rr) {
-            if (rr >= nrows) break;  // uniform across the CTA
-            uint32_t d[4];
-            {
-                // code i of the row at word 36 (i >> 6) + (i & 63) / 2 = i / 2 + 4 (i >> 6)
-                const uint32_t i = (lin0 & 63u) + t4;
-                const uint2    v = *reinterpret_cast<const uint2*>(rows[rr] + (i >> 1) + 4 * (i >> 6));
-                sm_decode2(v.x, d[0], d[1]);
-                sm_decode2(v.y, d[2], d[3]);
-            }
-            d[1] += d[0], d[2] += d[1], d[3] += d[2];
-            uint32_t v = d[3];
-            uint32_t u = __shfl_up_sync(kFull, v, 1);
-            if (q >= 1) v += u;
-            u = __shfl_up_sync(kFull, v, 2);
-            if (q >= 2) v += u;
-            const uint32_t ex = v - d[3];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[j] += d[j] + ex;
-            if (live)
-                *reinterpret_cast<float4*>(a.out + lin0 + 4 * tid) =
-                    make_float4((float)(int32_t)acc[0] * a.ebx2, (float)(int32_t)acc[1] * a.ebx2,
-                                (float)(int32_t)acc[2] * a.ebx2, (float)(int32_t)acc[3] * a.ebx2);
-            lin0 += a.x;
-        }
-        return;
-    }
-#pragma unroll 4
-    for (uint32_t rr = 0; rr < 16; ++rr) {
-        const uint32_t row = r0 + rr;
-        if (row >= a.y) break;  // uniform across the CTA
-        const uint32_t lin0 = row * a.x + c0;
-        uint32_t       d[4];
-        // threads past the window's end read the row's first codes (same alignment, in bounds,
-        // never stored; their values reach only higher quad positions, past the end too)
-        rb_read4<true>(rows[rr], (lin0 & 63u) + (live ? 4 * tid : 0u), d);
-        d[1] += d[0], d[2] += d[1], d[3] += d[2];
-        uint32_t v = d[3];
-        uint32_t u = __shfl_up_sync(kFull, v, 1);
-        if (q >= 1) v += u;
-        u = __shfl_up_sync(kFull, v, 2);
-        if (q >= 2) v += u;
-        const uint32_t ex = v - d[3];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] += d[j] + ex;
-        if (live) store4(a.out, lin0 + 4 * tid, c1 - col, acc, a.ebx2);
-    }
-}
-
-// ------------------------------------------- fused 2D decode, x % 16 == 0 --
-// Rows a multiple of 16 elements long: every 16-column tile row lies inside one 64-code
-// group (group and tile boundaries are both multiples of 16 in the linear index), so
-// phase 1 does the whole x direction.  Thread (row rr, j) decodes group glo(rr) + j, and for
-// each of its four tiles inside the window decodes the 16 codes, prefix-sums them serially
-// and writes the 16 partial sums as 32-bit words into the window's row (chunk c of 4 words
-// at c ^ ((c >> 4) & 7): the lanes' stores, 64 words apart, and phase 2's loads spread over
-// all banks).  Phase 2: thread t owns columns 4t..4t+3 -- a running sum over the band's
-// rows, (float)p * ebx2, coalesced stores; no shuffles, so threads past the window leave.
-constexpr uint32_t kW16 = 960;
-constexpr uint32_t kX16Smem = 16 * kW16 * 4;  // 16 rows x 960 partial sums
-
-__device__ __forceinline__ uint32_t x16_chunk(uint32_t c) { return c ^ ((c >> 4) & 7u); }
-
-__global__ void __launch_bounds__(256, 3) k_decompress2d_x16(const DecodeArgs a, uint32_t nwin)
-{
-    pdl_wait();
-    pdl_trigger();
-    extern __shared__ __align__(16) uint32_t xs[];  // [16][kW16] partial sums along x
-    const uint32_t tid = threadIdx.x;
-    const uint32_t bx = blockIdx.x % nwin, by = blockIdx.x / nwin;
-    const uint32_t c0 = bx * kW16, c1 = min(c0 + kW16, a.x);
-    const uint32_t r0 = by * 16;
-    {
-        const uint32_t rr = tid >> 4, j = tid & 15u, row = r0 + rr;
-        if (row < a.y) {
-            const uint32_t lin0 = row * a.x + c0, lin1 = row * a.x + c1;
-            const uint32_t g = (lin0 >> 6) + j;
-            if (g <= ((lin1 - 1) >> 6)) {
-                uint32_t w[32];
-                decode_group(a, g, w);
-                uint32_t* xr = xs + rr * kW16;
-#pragma unroll
-                for (uint32_t q = 0; q < 4; ++q) {
-                    const uint32_t e = g * 64 + q * 16;  // the tile row's first code
-                    if (e < lin0 || e >= lin1) continue;
-                    uint32_t v[16], acc = 0;
-#pragma unroll
-                    for (uint32_t k = 0; k < 8; ++k) {
-                        uint32_t d0, d1;
-                        sm_decode2(w[8 * q + k], d0, d1);
-                        acc += d0, v[2 * k] = acc;
-                        acc += d1, v[2 * k + 1] = acc;
-                    }
-                    const uint32_t c = (e - lin0) >> 2;  // first chunk of the tile row in the window row
-#pragma unroll
-                    for (uint32_t s = 0; s < 4; ++s)
-                        *reinterpret_cast<uint4*>(xr + 4 * x16_chunk(c + s)) =
-                            make_uint4(v[4 * s], v[4 * s + 1], v[4 * s + 2], v[4 * s + 3]);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    const uint32_t col = c0 + 4 * tid;
-    if (col >= c1) return;  // phase 2 has no shuffles or barriers
+    Pair           s0{0.0f, 0.0f}, s1{0.0f, 0.0f};  // sums along y of the 4 columns
     const uint32_t nrows = min(16u, a.y - r0);
-    const uint32_t* xp   = xs + 4 * x16_chunk(tid);
-    float*          out  = a.out + (size_t)r0 * a.x + col;
-    uint32_t        acc[4] = {0, 0, 0, 0};
+    uint32_t       lin0  = r0 * a.x + c0;  // first code of the window in row r0 + rr
+    // threads past the window's end read the row's first codes (same alignment, in bounds; their
+    // values reach only higher quad positions, past the end too, and are not stored)
+    const uint32_t t4 = live ? 4 * tid : 0u;
 #pragma unroll 4
     for (uint32_t rr = 0; rr < 16; ++rr) {
         if (rr >= nrows) break;  // uniform across the CTA
-        const uint4 p = *reinterpret_cast<const uint4*>(xp + rr * kW16);
-        acc[0] += p.x, acc[1] += p.y, acc[2] += p.z, acc[3] += p.w;
-        *reinterpret_cast<float4*>(out) = make_float4((float)(int32_t)acc[0] * a.ebx2, (float)(int32_t)acc[1] * a.ebx2,
-                                                      (float)(int32_t)acc[2] * a.ebx2, (float)(int32_t)acc[3] * a.ebx2);
-        out += a.x;
+        uint32_t       x01, x23;
+        const uint32_t i = (lin0 & 63u) + t4;
+        rb_read4<kAl>(rows[rr], i, x01, x23);
+        Pair d0, d1;
+        sums_x<4>(x01, x23, q, d0, d1);
+        s0 = add2(s0, d0), s1 = add2(s1, d1);
+        store_row<kAl>(a.out + lin0 + 4 * tid, (int32_t)(c1 - col), s0, s1, a.ebx2);
+        lin0 += a.x;
     }
-}
-
-// Resident CTAs of k_decompress2d_x16 on the current device (0 on error), cached per device;
-// the first call also opts the kernel in to its dynamic shared memory (above 48 KB).
-static uint32_t x16_wave()
-{
-    static std::atomic<uint32_t> cache[64];
-    int                          dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    std::atomic<uint32_t>* slot = (dev >= 0 && dev < 64) ? &cache[dev] : nullptr;
-    uint32_t               w    = slot ? slot->load(std::memory_order_acquire) : 0u;
-    if (w) return w;
-    int sms = 0, per_sm = 0;
-    if (cudaFuncSetAttribute(k_decompress2d_x16, cudaFuncAttributeMaxDynamicSharedMemorySize, kX16Smem) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_decompress2d_x16, 256, kX16Smem) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return 0;
-    }
-    w = (uint32_t)std::max(0, sms * per_sm);
-    if (slot && w) slot->store(w, std::memory_order_release);
-    return w;
 }
 
 // ------------------------------------------------------ fused 3D decode --
@@ -468,14 +519,24 @@ static uint32_t x16_wave()
 // shuffle), running sum along y within the plane, running sum along z in shared memory
 // (one 16-byte slot per thread and row: in registers they would spill), then the
 // stores.
+//
+// Bound by the latency of its phases at the 20 warps an SM the slabs leave (a thread per 4 columns
+// and 8 rows), then by instruction issue (50%).  GB300, event-timed, with the decode and the sums
+// of the 2D kernel and 128 threads a CTA, against a sign per code, integer sums and 256 threads:
+// 500x500x100 41.2 -> 31.1 us, 256x256x256 38.9 -> 24.3, 501x500x100 55.3 -> 42.6, 64x64x64 24.1
+// -> 14.4.  Decoding plane p + 1 by half the warps while the others sum plane p: 37.1 us.
 struct Brick3 {
     uint32_t w, q2, bands, g;  // window columns, column quads, bands per CTA, slots per row
     uint32_t nwin, nbgrp;      // windows along x, band groups along y
     uint32_t span, pg;         // span mode; slots per plane buffer
+    uint32_t t;                // threads
 };
 constexpr uint32_t kW3 = 960;
 
-__global__ void __launch_bounds__(256, 4) k_decompress3d(const DecodeArgs a, const Brick3 k)
+// kAl: x % 4 == 0 (every group of 4 columns is whole and aligned, in the buffers and in the field).
+// kT: threads.
+template <bool kSpan, bool kAl, uint32_t kT>
+__global__ void __launch_bounds__(kT, 768 / kT) k_decompress3d(const DecodeArgs a, const Brick3 k)
 {
     pdl_wait();
     pdl_trigger();
@@ -488,75 +549,76 @@ __global__ void __launch_bounds__(256, 4) k_decompress3d(const DecodeArgs a, con
     const uint32_t ys = yb0 * 8, ye = min(ys + 8 * k.bands, a.y);  // the CTA's rows
     const uint32_t band = tid / k.q2, cq = tid - band * k.q2;
     const uint32_t col = c0 + 4 * cq, ybase = ys + band * 8;
-    const bool     bandlive = band < k.bands && ybase < a.y;
+    // rows of this thread's band that lie in the field (0: none, or past the window)
+    const uint32_t nrow = band < k.bands && ybase < a.y && col < c1 ? min(8u, a.y - ybase) : 0u;
     // buffer words per plane (span) or per row
-    const uint32_t rowwords = (k.span ? k.pg : k.g) * 32;
-    const uint32_t ntask    = k.span ? 2 * k.pg : k.bands * 16 * k.g;
+    const uint32_t rowwords = (kSpan ? k.pg : k.g) * kSlotWords;
+    const uint32_t ntask    = kSpan ? 2 * k.pg : k.bands * 16 * k.g;
     // running sums along z, one 16-byte slot per thread and row of its band (after the row buffers)
-    uint4* zs = reinterpret_cast<uint4*>(rb3 + (k.span ? 2 * k.pg : k.bands * 16 * k.g) * 32) + tid;
+    float4* zs = reinterpret_cast<float4*>(rb3 + (kSpan ? 2 : k.bands * 16) * rowwords) + tid;
 #pragma unroll
-    for (int yy = 0; yy < 8; ++yy) zs[yy * 256] = make_uint4(0, 0, 0, 0);
+    for (uint32_t yy = 0; yy < 8; ++yy) zs[yy * kT] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
     for (uint32_t pz = 0; pz < 8; pz += 2) {
         if (z0 + pz >= a.z) break;  // uniform across the CTA
-        for (uint32_t task = tid; task < ntask; task += 256) {
-            uint32_t r, j, lin0, lin1;
-            if (k.span) {
-                r = task / k.pg, j = task - r * k.pg;
-                const uint32_t zz = z0 + pz + r;
-                if (zz >= a.z) continue;
-                lin0 = (zz * a.y + ys) * a.x, lin1 = (zz * a.y + ye) * a.x;
+        for (uint32_t t0 = 0; t0 < ntask; t0 += kT) {
+            const uint32_t task = t0 + tid;
+            uint32_t       r, j, zz, yv, len;
+            if (kSpan) {
+                r = task >= k.pg ? 1u : 0u, j = task - r * k.pg;
+                zz = z0 + pz + r, yv = ys, len = (ye - ys) * a.x;
             } else {
                 r = task / k.g, j = task - r * k.g;
-                const uint32_t zz = z0 + pz + ((r >> 3) & 1u), yv = ys + (r >> 4) * 8 + (r & 7u);
-                if (zz >= a.z || yv >= a.y) continue;
-                lin0 = (zz * a.y + yv) * a.x + c0, lin1 = lin0 + (c1 - c0);
+                zz = z0 + pz + ((r >> 3) & 1u), yv = ys + (r >> 4) * 8 + (r & 7u), len = c1 - c0;
             }
-            const uint32_t g = (lin0 >> 6) + j;
-            if (g > ((lin1 - 1) >> 6)) continue;
-            uint32_t w[32];
-            decode_group(a, g, w);
-            rb_put_group<false>(rb3 + r * rowwords, j, w);
+            const uint32_t lin0 = (zz * a.y + yv) * a.x + c0, g = (lin0 >> 6) + j;
+            const bool     valid = task < ntask && zz < a.z && yv < a.y && g <= ((lin0 + len - 1) >> 6);
+            uint32_t       w[32];
+            decode_deltas(a, g, valid, w);
+            if (valid) rb_put_group<!kAl>(rb3 + r * rowwords, j, w);
         }
         __syncthreads();
+#pragma unroll 1
         for (uint32_t p = 0; p < 2; ++p) {
             const uint32_t zz = z0 + pz + p;
             if (zz >= a.z) break;  // uniform across the CTA
-            const uint32_t pbase = ((zz * a.y + ys) * a.x) & ~63u;  // span mode: first slot's code
-            uint32_t       colacc[4] = {0, 0, 0, 0};
+            // threads without rows read the buffer's first codes, and rows past the band's end repeat
+            // its last: neither is stored or reaches a thread or row that is
+            const uint32_t  row0 = nrow ? (zz * a.y + ybase) * a.x + c0 : 0u;  // first code of the window
+            float*          out  = a.out + row0 + 4 * cq;
+            const uint32_t* rb   = rb3 + (kSpan ? p : (nrow ? band * 16 : 0u) + p * 8) * rowwords;
+            // span mode: from the plane's first slot
+            uint32_t i = kSpan ? row0 - (((zz * a.y + ys) * a.x) & ~63u) : row0;
+            if (!nrow) i = 0;
+            Pair s0{0.0f, 0.0f}, s1{0.0f, 0.0f};  // sums along y within the plane
 #pragma unroll
             for (uint32_t yy = 0; yy < 8; ++yy) {
-                const uint32_t yv   = ybase + yy;
-                const bool     live = bandlive && yv < a.y && col < c1;
-                const uint32_t lin0 = (zz * a.y + yv) * a.x + c0;
-                uint32_t       d[4] = {0, 0, 0, 0};
-                if (live) {
-                    if (k.span) rb_read4<false>(rb3 + p * rowwords, lin0 + 4 * cq - pbase, d);
-                    else rb_read4<false>(rb3 + (band * 16 + p * 8 + yy) * rowwords, (lin0 & 63u) + 4 * cq, d);
+                uint32_t x01, x23;
+                rb_read4<kAl>(rb, (kSpan ? i : i & 63u) + (nrow ? 4 * cq : 0u), x01, x23);
+                Pair d0, d1;
+                sums_x<2>(x01, x23, cq, d0, d1);
+                s0 = add2(s0, d0), s1 = add2(s1, d1);
+                const float4 z4 = zs[yy * kT];
+                const Pair   z0 = add2(Pair{z4.x, z4.y}, s0), z1 = add2(Pair{z4.z, z4.w}, s1);
+                zs[yy * kT]    = make_float4(z0.x, z0.y, z1.x, z1.y);
+                store_row<kAl>(out, yy < nrow ? (int32_t)(c1 - col) : 0, z0, z1, a.ebx2);
+                if (yy + 1 < nrow) {
+                    i += a.x, out += a.x;
+                    if (!kSpan) rb += rowwords;
                 }
-                d[1] += d[0], d[2] += d[1], d[3] += d[2];
-                const uint32_t u  = __shfl_up_sync(kFull, d[3], 1);
-                const uint32_t ex = (cq & 1u) ? u : 0u;
-                const uint4    z4 = zs[yy * 256];
-                uint32_t       zv[4] = {z4.x, z4.y, z4.z, z4.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    colacc[j] += d[j] + ex;
-                    zv[j] += colacc[j];
-                }
-                zs[yy * 256] = make_uint4(zv[0], zv[1], zv[2], zv[3]);
-                if (live) store4(a.out, lin0 + 4 * cq, c1 - col, zv, a.ebx2);
             }
         }
         __syncthreads();
     }
 }
 
-// Brick shape of the fused 3D path for a field of width x and height y.  Span mode
-// (whole rows) takes as many bands as keep both the compute threads (bands x q2) and the
-// pass's decode tasks (2 pg) within the CTA's 256 threads.
-static Brick3 brick3(uint32_t x, uint32_t y)
+// Brick shape of the fused 3D path for a field of width x and height y, with t threads.  Span mode
+// (whole rows) takes as many bands as keep both the compute threads (bands x q2) and the pass's
+// decode tasks (2 pg) within the CTA's threads.
+static Brick3 brick3(uint32_t x, uint32_t y, uint32_t t)
 {
     Brick3 k{};
+    k.t  = t;
     k.w  = std::min<uint32_t>(kW3, (x + 7) & ~7u);
     k.q2 = k.w / 4;
     k.g  = (k.w + 62) / 64 + 1;
@@ -564,29 +626,50 @@ static Brick3 brick3(uint32_t x, uint32_t y)
     const uint32_t nbands = (uint32_t)cdiv(y, 8);
     k.span = k.nwin == 1;
     if (k.span) {
-        k.bands = std::max(1u, std::min(256u / k.q2, nbands));
+        k.bands = std::max(1u, std::min(t / k.q2, nbands));
         for (;;) {
             // a plane's span is at most 8 bands x rows of x codes, starting anywhere in a group;
-            // rows' last quads read up to 3 codes past it
-            k.pg = (8 * k.bands * x + 66) / 64 + 1;
-            if (k.bands == 1 || 2 * k.pg <= 256) break;
+            // rows' last quads read up to 3 codes past it.  x % 8 == 0: where bands start, a
+            // group starts, in the first plane; planes of a multiple of 64 codes keep that
+            const uint32_t n = 8 * k.bands * x;
+            k.pg = x % 8 == 0 && (uint64_t)x * y % 64 == 0 ? (uint32_t)cdiv(n, 64) : (n + 66) / 64 + 1;
+            if (k.bands == 1 || 2 * k.pg <= t) break;
             --k.bands;
         }
     } else {
-        k.bands = std::max(1u, std::min({8u, 256u / k.q2, nbands}));
-        while (k.bands > 1 && k.bands * 16 * k.g * 128 > 48 * 1024) --k.bands;
+        k.bands = std::max(1u, std::min({8u, t / k.q2, nbands}));
+        while (k.bands > 1 && k.bands * 16 * k.g * kSlotWords * 4 > 48 * 1024) --k.bands;
     }
     k.nbgrp = (uint32_t)cdiv(nbands, k.bands);
     return k;
 }
 
-// Dynamic shared memory of a k_decompress3d CTA: the row buffers (span mode at most 2 x 122
-// slots, otherwise at most 48 KB) and the z sums (8 rows x 256 threads x 16 bytes).
+// 128 threads where they are used as well as 256 would be (within a tenth), since more and
+// smaller CTAs decode and sum at different times: 500x500x100 on GB300 33.4 -> 31.3 us; 256
+// where 128 leave a band's worth of threads idle (256x256x256 35.6 -> 31.0 us with 3 bands of 4).
+static Brick3 brick3(uint32_t x, uint32_t y)
+{
+    const Brick3 big = brick3(x, y, 256);
+    if (big.q2 > 128) return big;
+    const Brick3 k = brick3(x, y, 128);
+    return 2 * 10 * k.bands >= 9 * big.bands ? k : big;
+}
+
+// Dynamic shared memory of a k_decompress3d CTA: the row buffers (at most 48 KB) and the z sums
+// (8 rows x 16 bytes per thread).
 constexpr uint32_t kDecompress3dSmemMax = 48 * 1024 + 8 * 256 * 16;
 
 static uint32_t brick3_smem(const Brick3& k)
 {
-    return (k.span ? 2 * k.pg * 128 : k.bands * 16 * k.g * 128) + 8 * 256 * 16;
+    return (k.span ? 2 * k.pg : k.bands * 16 * k.g) * kSlotWords * 4 + 8 * k.t * 16;
+}
+
+using Decompress3d = void(const DecodeArgs, const Brick3);
+template <uint32_t kT>
+static Decompress3d* decompress3d(bool span, bool al)
+{
+    return span ? (al ? k_decompress3d<true, true, kT> : k_decompress3d<true, false, kT>)
+                : (al ? k_decompress3d<false, true, kT> : k_decompress3d<false, false, kT>);
 }
 
 // Above 48 KB a kernel's dynamic shared memory needs an opt-in, which is per device.
@@ -598,7 +681,10 @@ static cudaError_t allow_decompress3d_smem()
     if (e != cudaSuccess) return e;
     const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
     if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_decompress3d, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecompress3dSmemMax);
+    for (int v = 0; v < 8 && e == cudaSuccess; ++v) {
+        Decompress3d* f = v & 4 ? decompress3d<128>(v & 1, v & 2) : decompress3d<256>(v & 1, v & 2);
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecompress3dSmemMax);
+    }
     if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
     return e;
 }
@@ -697,21 +783,11 @@ __global__ void __launch_bounds__(kDecode1dWarps * 32) k_decompress1d(const Deco
 cudaError_t launch_decompress_fused(const DecodeArgs& a, cudaStream_t s)
 {
     const int nd = (a.z == 1 && a.y == 1) ? 1 : (a.z == 1 ? 2 : 3);
-    if (nd == 2 && a.x % 16 == 0) {
-        // the x-in-phase-1 kernel (3 CTAs/SM) when its grid is one resident wave: measured on
-        // GB300, cesm-like 3600x1800 (452 CTAs) 14.0 -> 12.2 us a launch (in 8-branch graphs,
-        // where it leaves less room to other branches' kernels, the same throughput);
-        // exafel-like 39200x388 (1025 CTAs: 2.25 waves against 1.35 for k_decompress2d at 5
-        // CTAs/SM) 20.4 us either way
-        const uint32_t nwin = (uint32_t)cdiv(a.x, kW16);
-        const uint32_t ctas = (uint32_t)(nwin * cdiv(a.y, 16));
-        if (ctas <= x16_wave()) return launch_pdl(k_decompress2d_x16, dim3(ctas), dim3(256), kX16Smem, s, a, nwin);
-    }
     if (nd == 2) {
         const uint32_t nwin = (uint32_t)cdiv(a.x, kW2);
         const uint32_t ctas = (uint32_t)(nwin * cdiv(a.y, 16));
-        if (a.x % 4 == 0) return launch_pdl(k_decompress2d<true>, dim3(ctas), dim3(256), 0, s, a, nwin);
-        return launch_pdl(k_decompress2d<false>, dim3(ctas), dim3(256), 0, s, a, nwin);
+        if (a.x % 4 == 0) return launch_pdl(k_decompress2d<true>, dim3(ctas), dim3(kT2), 0, s, a, nwin);
+        return launch_pdl(k_decompress2d<false>, dim3(ctas), dim3(kT2), 0, s, a, nwin);
     }
     if (nd == 3) {
         const cudaError_t e = allow_decompress3d_smem();
@@ -719,7 +795,9 @@ cudaError_t launch_decompress_fused(const DecodeArgs& a, cudaStream_t s)
         const Brick3   k    = brick3(a.x, a.y);
         if (brick3_smem(k) > kDecompress3dSmemMax) return cudaErrorInvalidConfiguration;
         const uint64_t ctas = (uint64_t)k.nwin * k.nbgrp * cdiv(a.z, 8);
-        return launch_pdl(k_decompress3d, dim3((uint32_t)ctas), dim3(256), brick3_smem(k), s, a, k);
+        Decompress3d*  f    = k.t == 128 ? decompress3d<128>(k.span != 0, a.x % 4 == 0)
+                                        : decompress3d<256>(k.span != 0, a.x % 4 == 0);
+        return launch_pdl(f, dim3((uint32_t)ctas), dim3(k.t), brick3_smem(k), s, a, k);
     }
     const uint32_t ntiles = a.nb + (a.tail ? 1u : 0u);
     return launch_pdl(k_decompress1d, dim3((uint32_t)cdiv(ntiles, kDecode1dWarps)), dim3(kDecode1dWarps * 32), 0, s,

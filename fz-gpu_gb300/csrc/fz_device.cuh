@@ -150,11 +150,11 @@ __device__ __forceinline__ uint32_t shr_mul(uint32_t x)
 // kMul: the shifts as multiplies, where the integer/logic pipe is the bound (decompression of
 // the exafel-like field on GB300 21.8 -> 21.3 us; the staged encode); the float path of the
 // encode, bound by instruction issue, keeps the shifts (27.1 -> 27.7 us with multiplies).
-template <bool kMul, int J, uint32_t M>
-__device__ __forceinline__ void swap_stage(uint32_t (&a)[32])
+template <bool kMul, int J, uint32_t M, int N>
+__device__ __forceinline__ void swap_stage(uint32_t (&a)[N])
 {
 #pragma unroll
-    for (int r = 0; r < 32; ++r) {
+    for (int r = 0; r < N; ++r) {
         if (r & J) continue;
         const uint32_t lo = a[r], hi = a[r + J];
         const uint32_t hs = kMul ? shl_mul<J>(hi) : hi << J;
@@ -185,6 +185,14 @@ __device__ __forceinline__ void transpose32(uint32_t (&a)[32])
     swap_stage<kMul, 4, 0x0F0F0F0Fu>(a);
     swap_stage<kMul, 2, 0x33333333u>(a);
     swap_stage<kMul, 1, 0x55555555u>(a);
+}
+
+// The four 8x8 bit blocks of 8 words transposed: bit 8 c + i of a[r] becomes bit 8 c + r of a[i].
+__device__ __forceinline__ void transpose8(uint32_t (&a)[8])
+{
+    swap_stage<true, 4, 0x0F0F0F0Fu>(a);
+    swap_stage<true, 2, 0x33333333u>(a);
+    swap_stage<true, 1, 0x55555555u>(a);
 }
 
 // ------------------------------------------------------ scan tile state --
