@@ -130,6 +130,8 @@ SIGNATURES = {
 def lib():
     """Load libfzgb300.so (fails loudly when it has not been built)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):
@@ -261,18 +263,16 @@ def compress(x, dims, eb, rel=True, mode=MODE_SIDECAR, ws=None, out=None, stream
     Returns the stream as a CUDA uint8 tensor trimmed to its size (``readback=True``,
     one sync), or the untrimmed output buffer (``readback=False``, no sync)."""
     import torch
-    x = x.contiguous().view(-1)
     if x.dtype != torch.float32 or not x.is_cuda:
         raise FzError("compress wants a CUDA float32 tensor", INVALID_ARG)
+    x = x.contiguous()
     n = x.numel()
-    cap = max_compressed_bytes(n, dims, mode)
     if out is None:
-        out = torch.empty(cap, dtype=torch.uint8, device=x.device)
+        out = torch.empty(max_compressed_bytes(n, dims, mode), dtype=torch.uint8, device=x.device)
     ws = _ws_for(ws, n)
     nbytes = C.c_uint64(0)
-    st = lib().fz_compress(ws.handle, C.c_void_p(x.data_ptr()), n, _dims(dims), float(eb),
-                           EB_REL if rel else EB_ABS, mode, C.c_void_p(out.data_ptr()), out.numel(),
-                           C.byref(nbytes) if readback else None, _stream_handle(stream))
+    st = lib().fz_compress(ws.handle, x.data_ptr(), n, _dims(dims), float(eb), EB_REL if rel else EB_ABS, mode,
+                           out.data_ptr(), out.numel(), C.byref(nbytes) if readback else None, _stream_handle(stream))
     _check("fz_compress", st)
     return out[: nbytes.value] if readback else out
 
@@ -286,8 +286,8 @@ def decompress(stream_t, header=None, out=None, ws=None, stream=None):
     if out is None:
         out = torch.empty(n, dtype=torch.float32, device=stream_t.device)
     ws = _ws_for(ws, n)
-    st = lib().fz_decompress(ws.handle, C.c_void_p(stream_t.data_ptr()), stream_t.numel(), C.byref(header),
-                             C.c_void_p(out.data_ptr()), out.numel(), _stream_handle(stream))
+    st = lib().fz_decompress(ws.handle, stream_t.data_ptr(), stream_t.numel(), C.byref(header), out.data_ptr(),
+                             out.numel(), _stream_handle(stream))
     _check("fz_decompress", st)
     return out
 

@@ -107,16 +107,9 @@ fz_status check_device(const fz_workspace* ws)
     return dev == ws->device ? FZ_SUCCESS : FZ_INVALID_ARG;
 }
 
-// Reads back the header and the sticky status word (syncs), clears the status.
-fz_status readback(fz_workspace* ws, const void* d_stream, cudaStream_t s, fz_header* h)
+// The status word's bits as a status; clears the word when any is set.
+fz_status take_status(fz_workspace* ws, uint32_t st, cudaStream_t s)
 {
-    cudaError_t e = cudaMemcpyAsync(ws->h_pinned, d_stream, 64, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ws->h_pinned + 64, ws->status, 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
-    std::memcpy(h, ws->h_pinned, 64);
-    uint32_t st;
-    std::memcpy(&st, ws->h_pinned + 64, 4);
     if (st) cudaMemsetAsync(ws->status, 0, 4, s);
     if (st & kStatusTimeout) return FZ_TIMEOUT;
     if (st & kStatusNonfinite) return FZ_NONFINITE_INPUT;
@@ -340,11 +333,7 @@ fz_status fz_workspace_status(fz_workspace* ws, fz_stream_t stream)
     if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
     uint32_t st;
     std::memcpy(&st, ws->h_pinned + 64, 4);
-    if (st) cudaMemsetAsync(ws->status, 0, 4, s);
-    if (st & kStatusTimeout) return FZ_TIMEOUT;
-    if (st & kStatusNonfinite) return FZ_NONFINITE_INPUT;
-    if (st & kStatusCorrupt) return FZ_CORRUPT_STREAM;
-    return FZ_SUCCESS;
+    return take_status(ws, st, s);
 }
 
 fz_status fz_compress(fz_workspace* ws, const float* d_in, uint64_t n, fz_dims dims, double eb,
@@ -408,7 +397,11 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     st = compress_args(d_in, n, dims, eb, eb_mode, mode, d_out, out_capacity, ws->status, L, a);
     if (st != FZ_SUCCESS) return st;
     a.state = ws->state, a.ticket = ws->tickets + 0, a.epoch = ws->epoch;
-    a.mirror = mirror;
+    // A size readback comes through the pinned mirror, which the last launch writes directly
+    // (pinned host memory is mapped): no copy of the header and of the status word after it
+    // (GB300, a pass among others: 3600x1800 with its size 73.3 -> 54.6 us, 128x128 both ways 126 ->
+    // 107).
+    a.mirror = mirror ? mirror : out_bytes ? reinterpret_cast<uint32_t*>(ws->h_pinned) : nullptr;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     // the field as a list of one: range launch (relative eb), encode launch (per-block
     // slots in the workspace scratch, one 4 KiB slot per shuffle block; chunk counts in the
@@ -453,10 +446,18 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     if (e != cudaSuccess) return map_err(e);
     if (ra) ra->done = J.ahead_nr != 0;
     if (out_bytes) {
+        if (mirror) e = cudaMemcpyAsync(ws->h_pinned, mirror, 68, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) {
+            *out_bytes = L.off_b;
+            return map_err(e, FZ_FAIL_GPU_MEMCPY);
+        }
         fz_header h;
-        st = readback(ws, d_out, s, &h);
+        uint32_t  bits;
+        std::memcpy(&h, ws->h_pinned, 64);
+        std::memcpy(&bits, ws->h_pinned + 64, 4);
         *out_bytes = L.off_b + 16ull * h.nnz;
-        return st;
+        return take_status(ws, bits, s);
     }
     return FZ_SUCCESS;
 }
@@ -578,9 +579,8 @@ fz_status fz_decompress_host(fz_workspace* ws, const void* h_stream, uint64_t st
     st = fz_decompress(ws, ws->d_stream, stream_bytes, &h, ws->d_field, ws->max_n, stream);
     if (st != FZ_SUCCESS) return st;
     e = cudaMemcpyAsync(h_out, ws->d_field, 4 * h.n, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
-    return fz_workspace_status(ws, stream);
+    return fz_workspace_status(ws, stream);  // (syncs: one wait for the field and the status)
 }
 
 fz_status fz_selftest_wait_timeout(fz_workspace* ws, fz_stream_t stream)
