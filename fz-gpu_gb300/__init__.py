@@ -329,7 +329,9 @@ def lorenzo_construct(data, dims, eb_abs, signum=False, quant=None, stream=None)
     import torch
     data = data.contiguous().view(-1)
     if quant is None:
-        quant = torch.zeros(data.numel(), dtype=torch.int16, device=data.device)
+        d = _dims(dims)
+        alloc = torch.empty if d.x * d.y * d.z == data.numel() else torch.zeros  # x*y*z codes are written
+        quant = alloc(data.numel(), dtype=torch.int16, device=data.device)
     sg = torch.zeros(data.numel(), dtype=torch.uint8, device=data.device) if signum else None
     st = lib().fz_lorenzo_construct(C.c_void_p(data.data_ptr()), C.c_void_p(quant.data_ptr()),
                                     C.c_void_p(sg.data_ptr()) if sg is not None else None,
@@ -360,7 +362,7 @@ def bitshuffle_flag(codes, stream=None):
     if n % 2:
         src = torch.zeros(n + 1, dtype=codes.dtype, device=codes.device)
         src[:n] = codes
-    out = torch.zeros(2 * words, dtype=codes.dtype, device=codes.device)
+    out = torch.empty(2 * words, dtype=codes.dtype, device=codes.device)  # all n written
     bit = torch.empty(nw, dtype=torch.int32, device=codes.device)
     byte = torch.empty(32 * nw, dtype=torch.int32, device=codes.device)
     st = lib().fz_bitshuffle_flag(C.c_void_p(src.data_ptr()), C.c_void_p(out.data_ptr()), n,

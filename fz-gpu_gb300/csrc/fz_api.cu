@@ -645,12 +645,12 @@ fz_status fz_scan_encode(fz_workspace* ws, const uint8_t* d_shuffled, const uint
     if (e != cudaSuccess) return map_err(e);
     if (nnz) {
         e = cudaMemcpyAsync(ws->h_pinned, ws->total, 4, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
+        st = fz_workspace_status(ws, stream);  // (syncs)
         uint32_t t;
         std::memcpy(&t, ws->h_pinned, 4);
         *nnz = t;
-        return fz_workspace_status(ws, stream);
+        return st;
     }
     return FZ_SUCCESS;
 }

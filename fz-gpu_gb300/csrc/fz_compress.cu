@@ -1800,7 +1800,9 @@ cudaError_t launch_bitshuffle_flag(const uint32_t* in, uint32_t* out, uint32_t n
 
 // fz_scan_encode: exclusive scan of M u32 flags (cub::DeviceScan::ExclusiveSum,
 // fz.cu:187-192) + total (fz.cu:194-201) + compaction (encodeDebug, fz.cu:49-59).
-// One warp per 256 flags, decoupled look-back across warps.
+// One warp per 256 flags, 8 warps to a tile, one decoupled look-back per tile.  Bound by its
+// round trips (flags, look-back, chunks).  A look-back per warp chained 8 times as many tiles:
+// 3600x1800 codes on GB300 29.6 -> 16 us.
 __global__ void __launch_bounds__(256) k_scan_encode(const uint8_t* __restrict__ shuffled,
                                                      const uint32_t* __restrict__ flags,
                                                      uint32_t n_codes, uint32_t m,
@@ -1809,7 +1811,7 @@ __global__ void __launch_bounds__(256) k_scan_encode(const uint8_t* __restrict__
                                                      uint32_t* status, uint32_t* total,
                                                      uint32_t* epoch_word)
 {
-    __shared__ uint32_t cta_tile, s_epoch;
+    __shared__ uint32_t cta_tile, s_epoch, s_cnt[8], s_pre[8];
     const uint32_t      lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         s_epoch = __ldcg(epoch_word);
@@ -1817,29 +1819,41 @@ __global__ void __launch_bounds__(256) k_scan_encode(const uint8_t* __restrict__
         cta_tile = take_ticket(ticket, epoch_word, gridDim.x).tile;
     }
     __syncthreads();
-    const uint32_t epoch = s_epoch;
-    const uint32_t t      = cta_tile * 8 + wid;
-    const uint32_t ntiles = m / 256;  // m = 32 * ceil(n/256), a multiple of 32; tiles of 256
-    const uint32_t ntl    = (m + 255) / 256;
-    if (t >= ntl) return;
-    (void)ntiles;
-    uint32_t bm[8], cnt = 0;
+    const uint32_t epoch = s_epoch, tile = cta_tile;
+    const uint32_t t     = tile * 8 + wid;  // the warp's 256 flags
+    const uint32_t ntl   = (m + 255) / 256;
+    uint32_t       bm[8], cnt = 0;
 #pragma unroll
     for (uint32_t i = 0; i < 8; ++i) {
-        const uint32_t idx = t * 256 + 32 * i + lane;
+        const uint32_t idx = t * 256 + 32 * i + lane;  // (m < 2^29)
         bm[i] = __ballot_sync(kFull, idx < m && flags[idx] != 0);
         cnt += __popc(bm[i]);
     }
-    uint32_t excl = 0, povf = 0;
-    if (t == 0) {
-        if (lane == 0) publish(state, 0, epoch, kFlagIncl, 0, cnt);
-    } else {
-        if (lane == 0) publish(state, t, epoch, kFlagAgg, 0, cnt);
-        lookback(state, t, epoch, status, excl, povf);
-        if (lane == 0) publish(state, t, epoch, kFlagIncl, 0, excl + cnt);
+    if (lane == 0) s_cnt[wid] = cnt;
+    __syncthreads();
+    if (wid == 0) {
+        const uint32_t c   = lane < 8 ? s_cnt[lane] : 0u;
+        const uint32_t tot = __reduce_add_sync(kFull, c);
+        uint32_t       excl = 0, povf = 0;
+        if (tile == 0) {
+            if (lane == 0) publish(state, 0, epoch, kFlagIncl, 0, tot);
+        } else {
+            if (lane == 0) publish(state, tile, epoch, kFlagAgg, 0, tot);
+            lookback(state, tile, epoch, status, excl, povf);
+            if (lane == 0) publish(state, tile, epoch, kFlagIncl, 0, excl + tot);
+        }
+        uint32_t inc = c;
+#pragma unroll
+        for (uint32_t o = 1; o < 8; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(kFull, inc, o);
+            if (lane >= o) inc += v;
+        }
+        if (lane < 8) s_pre[lane] = excl + inc - c;
     }
+    __syncthreads();
+    if (t >= ntl) return;
     const uint32_t lt       = lanemask_lt();
-    uint32_t       pre      = excl;
+    uint32_t       pre      = s_pre[wid];
     const uint64_t srcbytes = 2ull * n_codes;
 #pragma unroll
     for (uint32_t i = 0; i < 8; ++i) {

@@ -808,46 +808,59 @@ cudaError_t launch_decompress_fused(const DecodeArgs& a, cudaStream_t s)
 // ------------------------------------------------------------- recon --
 // 2D: a CTA covers 16 rows x 512 columns; lane owns 4 consecutive columns, lanes 4k..4k+3
 // one 16-column tile row.  Row prefix: serial over 4 + quad shuffle scan; column prefix:
-// running sum over the 16 rows.
+// running sum over the 16 rows.  Bound by latency: 8 rows' codes are loaded at a time (one
+// row at a time, 3600x1800 on GB300: 11.2 -> 8.1 us).
 __global__ void __launch_bounds__(128) k_recon2d(const ReconArgs a, uint32_t nwin)
 {
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const uint32_t c0   = (blockIdx.x % nwin) * 512 + wid * 128 + lane * 4;
     const uint32_t r0   = (blockIdx.x / nwin) * 16;
-    const uint32_t q    = lane & 3u;
+    const uint32_t q    = lane & 3u, nrows = min(16u, a.y - r0);
     const bool     vec  = (a.x % 4 == 0) && (c0 + 3 < a.x);
+    const size_t   base = (size_t)r0 * a.x + c0;
     uint32_t       acc[4] = {0, 0, 0, 0};
-    for (uint32_t rr = 0; rr < 16; ++rr) {
-        const uint32_t row = r0 + rr;
-        if (row >= a.y) break;  // uniform across the CTA
-        const size_t base = (size_t)row * a.x + c0;
-        uint32_t     d[4] = {0, 0, 0, 0};
-        if (vec) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2*>(a.codes + base));
-            sm_decode2(v.x, d[0], d[1]);
-            sm_decode2(v.y, d[2], d[3]);
-        } else {
+#pragma unroll 1
+    for (uint32_t h = 0; h < nrows; h += 8) {
+        uint2 w[8];  // 4 codes of each row
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (c0 + j < a.x) d[j] = sm_decode(a.codes[base + j]);
+        for (uint32_t rr = 0; rr < 8; ++rr) {
+            w[rr] = make_uint2(0, 0);
+            if (h + rr >= nrows) continue;  // uniform across the CTA
+            const uint16_t* src = a.codes + base + (size_t)(h + rr) * a.x;
+            if (vec) {
+                w[rr] = __ldg(reinterpret_cast<const uint2*>(src));
+            } else {
+                if (c0 < a.x) w[rr].x = src[0];
+                if (c0 + 1 < a.x) w[rr].x |= (uint32_t)src[1] << 16;
+                if (c0 + 2 < a.x) w[rr].y = src[2];
+                if (c0 + 3 < a.x) w[rr].y |= (uint32_t)src[3] << 16;
+            }
         }
-        d[1] += d[0], d[2] += d[1], d[3] += d[2];
-        uint32_t v = d[3];
-        uint32_t u = __shfl_up_sync(kFull, v, 1);
-        if (q >= 1) v += u;
-        u = __shfl_up_sync(kFull, v, 2);
-        if (q >= 2) v += u;
-        const uint32_t ex = v - d[3];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] += d[j] + ex;
-        if (vec) {
-            *reinterpret_cast<float4*>(a.out + base) =
-                make_float4((float)(int32_t)acc[0] * a.ebx2, (float)(int32_t)acc[1] * a.ebx2,
-                            (float)(int32_t)acc[2] * a.ebx2, (float)(int32_t)acc[3] * a.ebx2);
-        } else {
+        for (uint32_t rr = 0; rr < 8; ++rr) {
+            if (h + rr >= nrows) break;  // uniform across the CTA
+            uint32_t d[4];
+            sm_decode2(w[rr].x, d[0], d[1]);
+            sm_decode2(w[rr].y, d[2], d[3]);
+            d[1] += d[0], d[2] += d[1], d[3] += d[2];
+            uint32_t v = d[3];
+            uint32_t u = __shfl_up_sync(kFull, v, 1);
+            if (q >= 1) v += u;
+            u = __shfl_up_sync(kFull, v, 2);
+            if (q >= 2) v += u;
+            const uint32_t ex = v - d[3];
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (c0 + j < a.x) a.out[base + j] = (float)(int32_t)acc[j] * a.ebx2;
+            for (int j = 0; j < 4; ++j) acc[j] += d[j] + ex;
+            float* dst = a.out + base + (size_t)(h + rr) * a.x;
+            if (vec) {
+                *reinterpret_cast<float4*>(dst) =
+                    make_float4((float)(int32_t)acc[0] * a.ebx2, (float)(int32_t)acc[1] * a.ebx2,
+                                (float)(int32_t)acc[2] * a.ebx2, (float)(int32_t)acc[3] * a.ebx2);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (c0 + j < a.x) dst[j] = (float)(int32_t)acc[j] * a.ebx2;
+            }
         }
     }
 }
