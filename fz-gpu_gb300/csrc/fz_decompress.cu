@@ -695,55 +695,142 @@ static cudaError_t allow_decompress3d_smem()
 // x_lorenzo block), prefix-sums them serially, adds the quad's carry, and writes 64
 // floats through shared memory as coalesced 16-byte stores.  Codes at i%4 == 0 carry
 // their sign; the others take it from the sidecar sign bits (or are non-negative).
+//
+// Bound by the latency of its one chain per warp (bitmap, chunks, sums, stores), so by the warps
+// resident: 10 CTAs of 4 an SM, 48 registers and 4 KiB a warp.  GB300, event-timed, 2^25
+// elements at 1e-3 / 1e-4: 46.7 / 51.7 us with 32-bit sums and 8 KiB a warp, 42.7 / 49.4 with the
+// sums packed where they fit, 42.4 / 49.4, 38.7 / 45.1 and 37.0 / 43.4 with 6, 8 and 10 CTAs.
 constexpr int kDecode1dWarps = 4;
 
-// Word of prefix value j of lane l in a warp's shared buffer: the lane's 64 values as sixteen
-// 16-byte chunks, chunk c at position c ^ (l & 7), so that both the lanes' chunk stores here
-// and the output loop's chunk loads (16 lanes on one owner's 16 chunks) spread over all 32
-// banks.
-__device__ __forceinline__ uint32_t run1d_word(uint32_t l, uint32_t j) { return 64 * l + 4 * ((j >> 2) ^ (l & 7u)); }
+// A warp's shared buffer of 32 words a lane: 16-byte chunk c (of 8) of lane l at position c ^ (l & 7),
+// so that both the lanes' chunk stores and the output loops' loads (several lanes on one
+// owner's chunks) spread over all 32 banks.
+__device__ __forceinline__ uint32_t* chunk1d(uint32_t* sm, uint32_t l, uint32_t c) { return sm + 32 * l + 4 * (c ^ (l & 7u)); }
 
-// Lane-local inclusive prefix of the lane's 64 deltas into shared memory, four values per
-// 16-byte store; codes at i%4 == 0 carry their sign, the others take it from the sidecar
-// words s0, s1.  kCheck: only the first lim deltas count (the run ends past x*y*z).
-template <bool kCheck>
-__device__ __forceinline__ uint32_t run1d(const uint32_t (&w)[32], uint32_t s0, uint32_t s1, uint32_t lim,
-                                          uint32_t lane, uint32_t* sm)
+// Sums of the lane's deltas 32 h .. 32 h + 31 in 32 bits, from `acc` on; codes at i%4 == 0 carry
+// their sign, the others take it from the sidecar word s.  kStore: each sum into the lane's
+// words.  Only the run's first lim deltas count.
+template <int h, bool kStore>
+__device__ __forceinline__ uint32_t run1d(const uint32_t (&w)[32], uint32_t s, uint32_t lim, uint32_t lane, uint32_t acc,
+                                          uint32_t* sm)
 {
-    uint32_t acc = 0, q[4];
+    uint32_t q[4];
 #pragma unroll
-    for (int j = 0; j < 64; ++j) {
-        const uint32_t c   = (j & 1) ? (w[j >> 1] >> 16) : (w[j >> 1] & 0xFFFFu);
-        const uint32_t sgn = ((j < 32 ? s0 >> j : s1 >> (j - 32)) & 1u);
-        const uint32_t d   = (j & 3) == 0 ? sm_decode(c) : (sgn ? 0u - c : c);
-        acc += (!kCheck || (uint32_t)j < lim) ? d : 0u;
-        q[j & 3] = acc;
-        if ((j & 3) == 3) *reinterpret_cast<uint4*>(sm + run1d_word(lane, j)) = make_uint4(q[0], q[1], q[2], q[3]);
+    for (int i = 0; i < 32; ++i) {
+        const int      j = 32 * h + i;
+        const uint32_t c = (j & 1) ? (w[j >> 1] >> 16) : (w[j >> 1] & 0xFFFFu);
+        const uint32_t d = (j & 3) == 0 ? sm_decode(c) : ((s >> i) & 1u ? 0u - c : c);
+        acc += (uint32_t)j < lim ? d : 0u;
+        q[i & 3] = acc;
+        if (kStore && (i & 3) == 3) *reinterpret_cast<uint4*>(chunk1d(sm, lane, i >> 2)) = make_uint4(q[0], q[1], q[2], q[3]);
     }
     return acc;
 }
 
-__global__ void __launch_bounds__(kDecode1dWarps * 32) k_decompress1d(const DecodeArgs a)
+// Bits 0, 2, 4 ... of v as the low 16 bits.
+__device__ __forceinline__ uint32_t even_bits(uint32_t v)
+{
+    v &= 0x55555555u;
+    v = (v | (v >> 1)) & 0x33333333u;
+    v = (v | (v >> 2)) & 0x0F0F0F0Fu;
+    v = (v | (v >> 4)) & 0x00FF00FFu;
+    return (v | (v >> 8)) & 0xFFFFu;
+}
+
+// The packed path of k_decompress1d.  A lane's 64 deltas but the one that starts its tile (the
+// tile's first value itself, which goes into the lane's base) are below 2^9: their running sums
+// within the lane stay below 2^15, and two of them share a word.  w: the bit planes of the
+// lane's codes (low codes in 0..15, high ones in 16..31); s0, s1: the sidecar's signs;
+// base: the lane's first value's predecessor.  Leaves the sums plus 0x8000, two per word, in
+// the lanes' words of `sm`; false, with nothing done, where a lane of the warp has a larger
+// delta.
+__device__ __forceinline__ bool sums1d_packed(uint32_t (&w)[32], uint32_t s0, uint32_t s1, uint32_t lane, uint32_t* sm,
+                                              int32_t& base)
+{
+    const uint32_t first = (lane & 3u) == 0 ? 1u : 0u;  // low element 0 starts a tile
+    // plane 15: the sign of low codes at even words (i % 4 == 0), a magnitude bit elsewhere
+    const uint32_t big = ((w[9] | w[10] | w[11] | w[12] | w[13] | w[14] | (w[15] & 0xAAAAAAAAu)) & ~first) | w[25] | w[26] |
+                         w[27] | w[28] | w[29] | w[30] | w[31];
+    const uint32_t mid = ((w[7] | w[8]) & ~first) | w[23] | w[24];
+    if (__any_sync(kFull, big != 0)) return false;
+    uint32_t code = 0;  // the starting code
+#pragma unroll
+    for (int p = 15; p >= 0; --p) code = 2 * code + (w[p] & 1u);
+    const int32_t start = first ? (int32_t)sm_decode(code) : 0;
+    const uint32_t sl = ((w[15] & 0x55555555u) | ((even_bits(s0) | (even_bits(s1) << 16)) & 0xAAAAAAAAu)) & ~first;
+    const uint32_t sh = even_bits(s0 >> 1) | (even_bits(s1 >> 1) << 16);
+#pragma unroll
+    for (int p = 0; p < 9; ++p) w[p] &= ~first;
+    if (!__any_sync(kFull, mid != 0)) {  // below 2^7: as decode_deltas
+        uint32_t t[2][8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t s = h ? sh : sl;
+            uint32_t       c = s;
+#pragma unroll
+            for (int p = 0; p < 7; ++p) {
+                const uint32_t b = w[16 * h + p];
+                t[h][p]          = b ^ s ^ c;
+                c                = (b ^ s) & c;
+            }
+            t[h][7] = s ^ c;
+            transpose8(t[h]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            w[i]      = delta_bytes<0>(t[0][i], t[1][i]) ^ 0x80000000u;
+            w[8 + i]  = delta_bytes<1>(t[0][i], t[1][i]) ^ 0x80000000u;
+            w[16 + i] = delta_bytes<2>(t[0][i], t[1][i]) ^ 0x80000000u;
+            w[24 + i] = delta_bytes<3>(t[0][i], t[1][i]) ^ 0x80000000u;
+        }
+    } else {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t s = h ? sh : sl;
+            uint32_t       c = s;
+#pragma unroll
+            for (int p = 0; p < 9; ++p) {
+                const uint32_t b = w[16 * h + p];
+                w[16 * h + p]    = b ^ s ^ c;
+                c                = (b ^ s) & c;
+            }
+#pragma unroll
+            for (int p = 9; p < 16; ++p) w[16 * h + p] = s ^ c;  // the sign extended
+        }
+        w[15] = ~w[15];
+        transpose32<true>(w);
+    }
+    // w: deltas (d0 + 0x8000, d1) = d0 + 2^16 d1 + 0x8000 as an integer.  Times 2^16 + 1 that is
+    // (d0, d0 + d1), both plus 0x8000; the sum so far goes in before.
+    uint32_t h = 0x8000u;  // the sum so far plus 0x8000
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        w[j] = (w[j] + h - 0x8000u) * 65537u;
+        h    = w[j] >> 16;
+    }
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c)
+        *reinterpret_cast<uint4*>(chunk1d(sm, lane, c)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+    const int32_t run = (int32_t)h - 0x8000;
+    int32_t       v = run + start, u = __shfl_up_sync(kFull, v, 1);
+    if (lane & 3u) v += u;
+    u = __shfl_up_sync(kFull, v, 2);
+    if ((lane & 3u) >= 2) v += u;
+    base = v - run;
+    return true;
+}
+
+__global__ void __launch_bounds__(kDecode1dWarps * 32, 10) k_decompress1d(const DecodeArgs a)
 {
     pdl_wait();
     pdl_trigger();
-    __shared__ __align__(16) uint32_t smem[kDecode1dWarps][2048];
+    __shared__ __align__(16) uint32_t smem[kDecode1dWarps][kBlockWords];
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const uint32_t t    = blockIdx.x * kDecode1dWarps + wid;
     const uint32_t ntiles = a.nb + (a.tail ? 1u : 0u);
     if (t >= ntiles) return;  // warp-uniform
-    uint32_t* sm = smem[wid];
-    uint32_t  w[32];
-    if (t < a.nb) {
-        gather_block(a, t, lane, sm);
-        __syncwarp();
-#pragma unroll
-        for (uint32_t p = 0; p < 32; ++p) w[p] = sm[p * 32 + lane];
-        transpose32<true>(w);
-        __syncwarp();
-    } else {
-        decode_group(a, t * 32 + lane, w);  // tail: sidecar codes
-    }
+    uint32_t*       sm = smem[wid];
+    uint32_t        w[32];
     const uint32_t  e0 = t * kBlockCodes + lane * 64;
     const uint32_t* sb = (a.mode == 1) ? reinterpret_cast<const uint32_t*>(a.st + a.off_sign) : nullptr;
     uint32_t        s0 = 0, s1 = 0;
@@ -751,32 +838,65 @@ __global__ void __launch_bounds__(kDecode1dWarps * 32) k_decompress1d(const Deco
         s0 = __ldg(sb + (e0 >> 5));
         s1 = (e0 + 32 < a.n) ? __ldg(sb + (e0 >> 5) + 1) : 0u;
     }
+    if (t < a.nb) {
+        gather_block(a, t, lane, sm);
+        __syncwarp();
+#pragma unroll
+        for (uint32_t p = 0; p < 32; ++p) w[p] = sm[p * 32 + lane];
+        __syncwarp();
+        int32_t base;
+        if ((t + 1) * kBlockCodes <= a.nl && sums1d_packed(w, s0, s1, lane, sm, base)) {
+            // value = base + sum: each sum under the exponent of 2^23, less 2^23 + 2^15
+            const float c = (float)base - 8421376.0f;
+            __syncwarp();
+            float* out = a.out + (size_t)t * kBlockCodes + lane * 4;
+#pragma unroll 4
+            for (uint32_t i = 0; i < 16; ++i) {  // elements 128 i + 4 lane .. + 3: of lane `ow`
+                const uint32_t ow = 2 * i + (lane >> 4);
+                const float    co = __shfl_sync(kFull, c, ow);
+                const uint2    x  = *reinterpret_cast<const uint2*>(chunk1d(sm, ow, (lane & 15u) >> 1) + 2 * (lane & 1u));
+                const Pair     f{__uint_as_float(__byte_perm(x.x, 0x4B000000u, 0x7410)), __uint_as_float(__byte_perm(x.x, 0x4B000000u, 0x7432))};
+                const Pair     g{__uint_as_float(__byte_perm(x.y, 0x4B000000u, 0x7410)), __uint_as_float(__byte_perm(x.y, 0x4B000000u, 0x7432))};
+                store_row<true>(out + 128 * i, 4, add2(f, Pair{co, co}), add2(g, Pair{co, co}), a.ebx2);
+            }
+            return;
+        }
+        transpose32<true>(w);
+    } else {
+        decode_group(a, t * 32 + lane, w);  // tail: sidecar codes
+    }
     // elements of this lane's run inside x*y*z (all 64 except in the last block)
-    const uint32_t lim = a.nl > e0 ? a.nl - e0 : 0u;
-    const uint32_t acc = lim >= 64 ? run1d<false>(w, s0, s1, lim, lane, sm) : run1d<true>(w, s0, s1, lim, lane, sm);
+    const uint32_t lim  = a.nl > e0 ? a.nl - e0 : 0u;
+    const uint32_t half = run1d<0, true>(w, s0, lim, lane, 0u, sm);
+    const uint32_t acc  = run1d<1, false>(w, s1, lim, lane, half, sm);
     // carry across the 4 lanes of each 256-element block
     uint32_t v = acc, u = __shfl_up_sync(kFull, v, 1);
     if (lane & 3u) v += u;
     u = __shfl_up_sync(kFull, v, 2);
     if ((lane & 3u) >= 2) v += u;
     const uint32_t ex = v - acc;
-    __syncwarp();
-    // write: pass i covers elements i*128 .. i*128+127 of the block; lane owns 4
-    float* out = a.out + (size_t)t * kBlockCodes;
-    for (uint32_t i = 0; i < 16; ++i) {
-        const uint32_t el = i * 128 + lane * 4;   // element within the block
-        const uint32_t ow = el >> 6, j0 = el & 63u;  // owning lane, index in its run
-        const uint32_t exo = __shfl_sync(kFull, ex, ow);
-        const uint4    pv  = *reinterpret_cast<const uint4*>(sm + run1d_word(ow, j0));  // j0 % 4 == 0
-        const float    f[4] = {(float)(int32_t)(pv.x + exo) * a.ebx2, (float)(int32_t)(pv.y + exo) * a.ebx2,
-                               (float)(int32_t)(pv.z + exo) * a.ebx2, (float)(int32_t)(pv.w + exo) * a.ebx2};
-        const uint32_t e = t * kBlockCodes + el;
-        if (e + 3 < a.nl) {
-            *reinterpret_cast<float4*>(out + el) = make_float4(f[0], f[1], f[2], f[3]);
-        } else {
+    // write, half a run at a time: pass i covers 32 elements of the runs of lanes 4 i .. 4 i + 3
+#pragma unroll 1
+    for (uint32_t h = 0; h < 2; ++h) {
+        __syncwarp();
+        if (h) {
+            run1d<1, true>(w, s1, lim, lane, half, sm);
+            __syncwarp();
+        }
+        for (uint32_t i = 0; i < 8; ++i) {
+            const uint32_t ow  = 4 * i + (lane >> 3);
+            const uint32_t exo = __shfl_sync(kFull, ex, ow);
+            const uint4    pv  = *reinterpret_cast<const uint4*>(chunk1d(sm, ow, lane & 7u));
+            const float    f[4] = {(float)(int32_t)(pv.x + exo) * a.ebx2, (float)(int32_t)(pv.y + exo) * a.ebx2,
+                                   (float)(int32_t)(pv.z + exo) * a.ebx2, (float)(int32_t)(pv.w + exo) * a.ebx2};
+            const uint32_t e = t * kBlockCodes + 64 * ow + 32 * h + 4 * (lane & 7u);
+            if (e + 3 < a.nl) {
+                __stcs(reinterpret_cast<float4*>(a.out + e), make_float4(f[0], f[1], f[2], f[3]));
+            } else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (e + k < a.nl) out[el + k] = f[k];
+                for (int k = 0; k < 4; ++k)
+                    if (e + k < a.nl) a.out[e + k] = f[k];
+            }
         }
     }
 }

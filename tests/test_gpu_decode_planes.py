@@ -1,6 +1,6 @@
 """The fused decompression kernels against the oracle, bit for bit, where their decode changes
-method: deltas around the 2^7 below which planes 7..14 are not fetched (per warp), deltas up to
-the code limit, rows whose codes start anywhere in a 4-code group, windows and whole-row spans
+method: deltas around the 2^7 below which planes 7..14 are not fetched (per warp), in 1D around
+the 2^9 below which sums are packed, deltas up to the code limit, rows whose codes start anywhere in a 4-code group, windows and whole-row spans
 around their limits, bands and slabs cut short by the field's end, and tails in the sidecar."""
 import numpy as np
 import pytest
@@ -24,7 +24,7 @@ def ws(fz):
 def test_decode_magnitudes(fz, oracle, ws, dims, extra):
     n = dims[0] * dims[1] * dims[2] + extra
     rng = np.random.default_rng(n)
-    for top, share in ((3, 1.0), (31, 1.0), (127, 1.0), (128, 1.0), (5000, 0.001), (16000, 0.02), (32767, 0.3)):
+    for top, share in ((3, 1.0), (31, 1.0), (63, 1.0), (65, 1.0), (127, 1.0), (128, 1.0), (255, 1.0), (257, 1.0), (5000, 0.001), (16000, 0.02), (32767, 0.3)):
         # values whose deltas are mostly small and reach `top` (and beyond it, in sums of neighbours)
         data = np.where(rng.random(n) < share, rng.integers(-top, top + 1, n), rng.integers(-1, 2, n)).astype(np.float32)
         for mode in (0, 1):
