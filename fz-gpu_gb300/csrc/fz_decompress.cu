@@ -525,7 +525,8 @@ __global__ void __launch_bounds__(kT2, 4) k_decompress2d(const DecodeArgs a, uin
 // and 8 rows), then by instruction issue (50%).  GB300, event-timed, with the decode and the sums
 // of the 2D kernel and 128 threads a CTA, against a sign per code, integer sums and 256 threads:
 // 500x500x100 41.2 -> 31.1 us, 256x256x256 38.9 -> 24.3, 501x500x100 55.3 -> 42.6, 64x64x64 24.1
-// -> 14.4.  Decoding plane p + 1 by half the warps while the others sum plane p: 37.1 us.
+// -> 14.4; with both planes of a pass in one loop over the rows 30.2 -> 28.5, 23.3 -> 22.4, 42.5 ->
+// 39.5 and 14.4 -> 12.5.  Decoding plane p + 1 by half the warps while the others sum plane p: 37.1.
 struct Brick3 {
     uint32_t w, q2, bands, g;  // window columns, column quads, bands per CTA, slots per row
     uint32_t nwin, nbgrp;      // windows along x, band groups along y
@@ -579,34 +580,41 @@ __global__ void __launch_bounds__(kT, 768 / kT) k_decompress3d(const DecodeArgs 
             if (valid) rb_put_group<!kAl>(rb3 + r * rowwords, j, w);
         }
         __syncthreads();
-#pragma unroll 1
-        for (uint32_t p = 0; p < 2; ++p) {
-            const uint32_t zz = z0 + pz + p;
-            if (zz >= a.z) break;  // uniform across the CTA
-            // threads without rows read the buffer's first codes, and rows past the band's end repeat
-            // its last: neither is stored or reaches a thread or row that is
-            const uint32_t  row0 = nrow ? (zz * a.y + ybase) * a.x + c0 : 0u;  // first code of the window
-            float*          out  = a.out + row0 + 4 * cq;
-            const uint32_t* rb   = rb3 + (kSpan ? p : (nrow ? band * 16 : 0u) + p * 8) * rowwords;
-            // span mode: from the plane's first slot
-            uint32_t i = kSpan ? row0 - (((zz * a.y + ys) * a.x) & ~63u) : row0;
-            if (!nrow) i = 0;
-            Pair s0{0.0f, 0.0f}, s1{0.0f, 0.0f};  // sums along y within the plane
-#pragma unroll
-            for (uint32_t yy = 0; yy < 8; ++yy) {
-                uint32_t x01, x23;
-                rb_read4<kAl>(rb, (kSpan ? i : i & 63u) + (nrow ? 4 * cq : 0u), x01, x23);
-                Pair d0, d1;
-                sums_x<2>(x01, x23, cq, d0, d1);
-                s0 = add2(s0, d0), s1 = add2(s1, d1);
-                const float4 z4 = zs[yy * kT];
-                const Pair   z0 = add2(Pair{z4.x, z4.y}, s0), z1 = add2(Pair{z4.z, z4.w}, s1);
-                zs[yy * kT]    = make_float4(z0.x, z0.y, z1.x, z1.y);
-                store_row<kAl>(out, yy < nrow ? (int32_t)(c1 - col) : 0, z0, z1, a.ebx2);
-                if (yy + 1 < nrow) {
-                    i += a.x, out += a.x;
-                    if (!kSpan) rb += rowwords;
-                }
+        // both planes of the pass in one loop over the rows: two independent chains, and the sums
+        // along z read and written once.  Threads without rows read the buffers' first codes, and
+        // rows past the band's end repeat its last: neither is stored or reaches a thread or row
+        // that is; a second plane past the slab's end is summed (nothing follows) and not stored
+        const uint32_t  zz   = z0 + pz;
+        const uint32_t  plane = a.x * a.y;
+        const uint32_t  row0 = nrow ? (zz * a.y + ybase) * a.x + c0 : 0u;  // first code of the window
+        const bool      two  = zz + 1 < a.z;
+        float*          out  = a.out + row0 + 4 * cq;
+        const uint32_t* rb   = rb3 + (kSpan ? 0u : (nrow ? band * 16 : 0u) * rowwords);
+        const uint32_t* rc   = rb + (kSpan ? 1u : 8u) * rowwords;
+        // span mode: from the planes' first slots
+        const uint32_t f0 = (zz * a.y + ys) * a.x;
+        uint32_t       i = kSpan ? row0 - (f0 & ~63u) : row0, k1 = kSpan ? row0 + plane - ((f0 + plane) & ~63u) : row0 + plane;
+        if (!nrow) i = 0, k1 = 0;
+        Pair s0{0.0f, 0.0f}, s1{0.0f, 0.0f}, t0{0.0f, 0.0f}, t1{0.0f, 0.0f};  // sums along y
+#pragma unroll 8
+        for (uint32_t yy = 0; yy < 8; ++yy) {
+            uint32_t x01, x23, y01, y23;
+            rb_read4<kAl>(rb, (kSpan ? i : i & 63u) + (nrow ? 4 * cq : 0u), x01, x23);
+            rb_read4<kAl>(rc, (kSpan ? k1 : k1 & 63u) + (nrow ? 4 * cq : 0u), y01, y23);
+            const float4 z4 = zs[yy * kT];
+            Pair d0, d1, e0, e1;
+            sums_x<2>(x01, x23, cq, d0, d1);
+            sums_x<2>(y01, y23, cq, e0, e1);
+            s0 = add2(s0, d0), s1 = add2(s1, d1);
+            t0 = add2(t0, e0), t1 = add2(t1, e1);
+            Pair q0 = add2(Pair{z4.x, z4.y}, s0), q1 = add2(Pair{z4.z, z4.w}, s1);
+            store_row<kAl>(out, yy < nrow ? (int32_t)(c1 - col) : 0, q0, q1, a.ebx2);
+            q0 = add2(q0, t0), q1 = add2(q1, t1);
+            zs[yy * kT] = make_float4(q0.x, q0.y, q1.x, q1.y);
+            store_row<kAl>(out + plane, two && yy < nrow ? (int32_t)(c1 - col) : 0, q0, q1, a.ebx2);
+            if (yy + 1 < nrow) {
+                i += a.x, k1 += a.x, out += a.x;
+                if (!kSpan) rb += rowwords, rc += rowwords;
             }
         }
         __syncthreads();
