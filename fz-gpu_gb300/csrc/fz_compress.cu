@@ -32,9 +32,6 @@
 #ifndef FZ_BLOCK3D_UNROLL
 #define FZ_BLOCK3D_UNROLL 2
 #endif
-#ifndef FZ_ENCODE_CTAS
-#define FZ_ENCODE_CTAS 4
-#endif
 #ifndef FZ_RANGE_CTAS
 #define FZ_RANGE_CTAS 5
 #endif
@@ -766,17 +763,22 @@ __device__ void write_header(const CompressArgs& a, const EbInfo& e, uint32_t fl
 
 // Phase C of shuffle block t: lane g holds the bit planes of group g's codes (the transposed
 // words); the shuffled image into the warp's buffer `sm`, the chunk flags as 8 ballots (=
-// bitmap words 8t..8t+7, stored) and the chunk count.  c: chunks lane + 32 i.
+// bitmap words 8t..8t+7, stored) and the chunk count.  c: chunks lane + 32 i.  kBytes: planes
+// 8..14 are zero, and chunks of planes 8..11 neither written nor looked at.
+template <bool kBytes>
 __device__ __forceinline__ void flag_block(const CompressArgs& a, uint32_t t, uint32_t lane, const uint32_t (&w)[32],
                                            uint32_t* sm, uint32_t (&bm)[8], uint32_t& cnt, uint4 (&c)[8])
 {
     // shuffled image S[p*32 + g] = w[p] (bitshuffleAndBitflag's out, fz.cu:82)
 #pragma unroll
-    for (uint32_t p = 0; p < 32; ++p) sm[p * 32 + lane] = w[p];
+    for (uint32_t p = 0; p < 32; ++p)
+        if (!kBytes || (p & 12u) != 8u) sm[p * 32 + lane] = w[p];
     __syncwarp();
     // chunk c = lane + 32 i; ballot i is bitmap word 8t+i
 #pragma unroll
     for (uint32_t i = 0; i < 8; ++i) {
+        bm[i] = 0;
+        if (kBytes && (i & 3u) == 2u) continue;
         c[i]  = *reinterpret_cast<const uint4*>(sm + (lane + 32 * i) * 4);
         bm[i] = __ballot_sync(kFull, (c[i].x | c[i].y | c[i].z | c[i].w) != 0);
         cnt += __popc(bm[i]);
@@ -861,7 +863,7 @@ __device__ __forceinline__ void compute_block(const CompressArgs& a, const Geo& 
         transpose32(w);
         __syncwarp();
         uint4 c[8];
-        flag_block(a, t, lane, w, sm, bm, cnt, c);
+        flag_block<false>(a, t, lane, w, sm, bm, cnt, c);
     } else if (t == a.nb && a.n > base) {
         // ---- tail block: n mod 2048 codes, never shuffled (fz.cu:173) ----
         const uint32_t tail = a.n - base;
@@ -1040,7 +1042,10 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_compress(const Compr
 // A single field is a list of one whose job is a kernel parameter.  The stream bytes equal
 // the single-pass look-back kernel's.
 constexpr uint32_t kCompactBlocks = 32;   // shuffle blocks per compaction item
-constexpr int      kEncodeCtas    = FZ_ENCODE_CTAS;  // CTAs per SM the encode kernels are built for
+// CTAs per SM the encode kernels are built for: the 3D variants spill at 64 registers (500x500x100
+// on GB300 34.6 us with 4 CTAs, 33.0 with 3; 39200x388 20.8 and 21.7).
+template <int ND>
+constexpr int kEncodeCtas = ND == 3 ? 3 : 4;
 static_assert(kItemCodes == kCompressWarps * kBlockCodes, "an encode item is a CTA's blocks");
 
 
@@ -1139,6 +1144,7 @@ constexpr uint32_t kCountPar = 1u << 31;
 
 // Block t's non-zero chunks (lane's: lane + 32 k) into its slot, its count into counts[] and
 // the group sums.
+template <bool kBytes = false>
 __device__ __forceinline__ void emit_block(const FieldJob& J, uint32_t t, uint32_t lane, const uint4 (&c)[8],
                                            const uint32_t (&bm)[8], uint32_t cnt, uint32_t par)
 {
@@ -1147,6 +1153,7 @@ __device__ __forceinline__ void emit_block(const FieldJob& J, uint32_t t, uint32
     uint32_t       pre = 0;
 #pragma unroll
     for (uint32_t k = 0; k < 8; ++k) {
+        if (kBytes && (k & 3u) == 2u) continue;
         if ((bm[k] >> lane) & 1u) S[pre + __popc(bm[k] & lt)] = c[k];
         pre += __popc(bm[k]);
     }
@@ -1223,11 +1230,28 @@ __device__ __forceinline__ void packed_block(const FieldJob& J, uint32_t t, uint
     const CompressArgs& a    = J.a;
     const uint8_t*      st   = reinterpret_cast<const uint8_t*>(smem);
     const uint32_t      i0   = halo + (wid * 32 + lane) * 64;
-    uint32_t            w[32], bm[8], cnt = 0, slow, shigh;
+    uint32_t            w[32], bm[8], cnt = 0, slow, shigh, wide = kFull;
     if constexpr (ND == 1) packed_deltas1(st, i0, lane, w);
-    else packed_deltas<ND, kRow, kX, kNarrow>(st, i0, t * kBlockCodes + lane * 64, a.x, a.y, a.xy, a.dx, a.dxy, w);
+    else wide = packed_deltas<ND, kRow, kX, kNarrow>(st, i0, t * kBlockCodes + lane * 64, a.x, a.y, a.xy, a.dx, a.dxy, w);
     __syncthreads();
     uint32_t* sm = smem + wid * kBlockWords;
+    uint4     c[8];
+    if (ND != 1 && t != a.nb && !__any_sync(kFull, (wide & 0xFF00FF00u) != 0)) {
+        // no delta of the block needs more than 8 bits (a compressible stream's deltas mostly do
+        // not, but where tile corners hold values)
+        uint32_t v[32], lo[8], hi[8];
+        byte_planes(w, lo, hi, slow, shigh);
+#pragma unroll
+        for (int p = 0; p < 8; ++p) v[p] = lo[p], v[8 + p] = 0u, v[16 + p] = hi[p], v[24 + p] = 0u;
+        v[15] = slow, v[31] = shigh;
+        flag_block<true>(a, t, lane, v, sm, bm, cnt, c);
+        emit_block<true>(J, t, lane, c, bm, cnt, par);
+        return;
+    }
+    if (ND != 1) {
+#pragma unroll
+        for (int k = 0; k < 32; ++k) w[k] -= kBias2s - kBias2;
+    }
     if (t == a.nb) {  // (warp-uniform)
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k)
@@ -1241,8 +1265,7 @@ __device__ __forceinline__ void packed_block(const FieldJob& J, uint32_t t, uint
     if (ND == 1 && a.mode == 1)  // the group's 64 signs, in element order
         *reinterpret_cast<uint2*>(a.out + a.off_sign + (size_t)t * (kBlockCodes / 8) + 8 * lane) =
             make_uint2(spread16(slow & 0xFFFFu) | (spread16(shigh & 0xFFFFu) << 1), spread16(slow >> 16) | (spread16(shigh >> 16) << 1));
-    uint4 c[8];
-    flag_block(a, t, lane, w, sm, bm, cnt, c);
+    flag_block<false>(a, t, lane, w, sm, bm, cnt, c);
     emit_block(J, t, lane, c, bm, cnt, par);
 }
 
@@ -1495,7 +1518,7 @@ __device__ __forceinline__ void range_ahead(const FieldJob& J, uint32_t total)
 }
 
 template <int ND, bool kList>
-__global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas)
+__global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas<ND>)
     k_encode_fields(const FieldJob* __restrict__ jobs, const Segment* __restrict__ segs, uint32_t nseg, uint32_t total,
                     const __grid_constant__ FieldJob one)
 {

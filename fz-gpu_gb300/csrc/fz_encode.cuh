@@ -19,13 +19,16 @@
 //    d = T - T(left), zero outside the tile, two elements per instruction.  The signs become
 //    sign-magnitude after the transpose, a bit plane at a time.
 //
+// Blocks whose deltas fit 8 bits transpose bytes (byte_planes) instead of 16-bit words.
+//
 // What bounds it: the float path is bound by instruction issue (3D: 3690 warp instructions per
-// 2048-element block, each value quantised for every stencil role it has); this one issues 1700
+// 2048-element block, each value quantised for every stencil role it has); this one issues 1500
 // and its staging phase runs at the copy bandwidth.  Encode launches on GB300, relative bound
-// 1e-3, CUDA events around each launch, float path -> this one: 500x500x100 57.9 -> 36.6 us,
-// 501x500x100 81.7 -> 39.6, 39200x388 26.9 -> 24.6, 3600x1800 16.4 -> 14.4, 3601x1801 19.6 ->
-// 14.5, 2^25 46.9 -> 35.0.  4 CTAs of 8 warps an SM (64 registers, 34-43 KB); 3 CTAs of 80
-// registers measured the same.
+// 1e-3, CUDA events around each launch, float path -> this one: 500x500x100 57.9 -> 33.0 us,
+// 501x500x100 81.7 -> 38.3, 39200x388 26.9 -> 20.8, 8192x8192 97.1 -> 74.5, 3600x1800 16.4 ->
+// 14.4, 3601x1801 19.6 -> 14.4, 2^25 46.9 -> 34.5 (the last at the DRAM's rate: field and slots
+// exceed the L2).  Of that the byte planes gave 39200x388 23.6 -> 20.8, 500x500x100 37.2 -> 33.0.
+// Items of 4 blocks, 5 CTAs an SM and deeper batches of loads measured the same or slower.
 #pragma once
 
 #include "fz_internal.h"
@@ -42,6 +45,7 @@ constexpr uint32_t kStageSlot = 136;  // bytes of 64 staged elements
 // staging.
 constexpr uint32_t kHaloRow = 4096;
 constexpr uint32_t kBias2   = 0x80008000u;
+constexpr uint32_t kBias2s  = 0x80808080u;  // of the deltas: a half's high byte is 0x80 where -128 <= d < 128
 // Bound on the 16-bit path's magnitudes (a little below 2^15: the bounds are computed in
 // float).
 constexpr float kPackedMax = 32600.0f;
@@ -296,9 +300,9 @@ __device__ __forceinline__ void low_halves(uint32_t k, uint32_t& m0, uint32_t& m
     m1 = k <= 2 ? 0u : k == 3 ? 0xFFFFu : kFull;
 }
 
-// The 64 deltas (biased by 0x8000) of the lane's group of the block that starts at element
-// e0 - 64 lane, two per word, from the staged differences; i0 = staged index of e0.
-// 1D: 256-element tiles, only the left neighbour.
+// The 64 deltas of the lane's group of the block that starts at element e0 - 64 lane, two per
+// word, biased, from the staged differences; i0 = staged index of e0.
+// 1D: 256-element tiles, only the left neighbour; biased by 0x8000.
 __device__ __forceinline__ void packed_deltas1(const uint8_t* st, uint32_t i0, uint32_t lane, uint32_t (&w)[32])
 {
     const uint8_t* pc = st + (i0 >> 6) * kStageSlot;  // i0 % 64 == 0
@@ -313,13 +317,14 @@ __device__ __forceinline__ void packed_deltas1(const uint8_t* st, uint32_t i0, u
     }
 }
 
-// 2D and 3D.  kRow: subtract the row above (2D with the row staged, 3D).  kX: x % 4 where the row
+// 2D and 3D; biased by 0x8080; returns nonzero bits under 0xFF00FF00 where a delta does not fit 8
+// bits.  kRow: subtract the row above (2D with the row staged, 3D).  kX: x % 4 where the row
 // above is read (0, 2, or 1 for any odd x).  Rows of 64 elements and more end at most once in
 // a lane's 64: that end, inside a group of 4, is behind a test of a warp-wide mask, and which
 // elements start a tile row -- every 16th (8th) -- is kept as masks.  kNarrow (8 <= x < 64):
 // both are found for each group.
 template <int ND, bool kRow, int kX, bool kNarrow>
-__device__ __forceinline__ void packed_deltas(const uint8_t* st, uint32_t i0, uint32_t e0, uint32_t x, uint32_t y,
+__device__ __forceinline__ uint32_t packed_deltas(const uint8_t* st, uint32_t i0, uint32_t e0, uint32_t x, uint32_t y,
                                               uint32_t xy, const FastDiv& dx, const FastDiv& dxy, uint32_t (&w)[32])
 {
     constexpr uint32_t tw = ND == 2 ? 15u : 7u;  // tile width - 1
@@ -346,7 +351,7 @@ __device__ __forceinline__ void packed_deltas(const uint8_t* st, uint32_t i0, ui
     starts((0u - col) & tw);
     // the row above: halves h0 + k of the staging slots from ra on, h0 the same in every lane
     const uint32_t h0 = (0u - x) & 63u;
-    uint32_t       last = 0, tp;  // tp: T of element e0 - 1 in the high half
+    uint32_t       last = 0, wide = 0, tp;  // tp: T of element e0 - 1 in the high half
     const uint8_t* ra = nullptr;
     auto word = [&](uint32_t h) { return *reinterpret_cast<const uint32_t*>(ra + 2 * h + ((h & 64u) >> 3)); };
     {
@@ -405,10 +410,12 @@ __device__ __forceinline__ void packed_deltas(const uint8_t* st, uint32_t i0, ui
             t01 = t01 - pick(m0, a0, kBias2) + kBias2;
             t23 = t23 - pick(m1, a1, kBias2) + kBias2;
         }
-        w[2 * j]     = t01 - pick(s0, kBias2, __byte_perm(tp, t01, 0x5432)) + kBias2;
-        w[2 * j + 1] = t23 - (kX == 0 ? __byte_perm(t01, t23, 0x5432) : pick(s1, kBias2, __byte_perm(t01, t23, 0x5432))) + kBias2;
-        tp           = t23;
+        w[2 * j]     = t01 - pick(s0, kBias2, __byte_perm(tp, t01, 0x5432)) + kBias2s;
+        w[2 * j + 1] = t23 - (kX == 0 ? __byte_perm(t01, t23, 0x5432) : pick(s1, kBias2, __byte_perm(t01, t23, 0x5432))) + kBias2s;
+        wide |= (w[2 * j] ^ kBias2) | (w[2 * j + 1] ^ kBias2);
+        tp = t23;
     }
+    return wide;
 }
 
 // Bit planes of 32 words of two biased deltas (after the transpose: plane p of the low
@@ -444,6 +451,35 @@ __device__ __forceinline__ uint32_t sign_mag2(uint32_t e, uint32_t& neg)
     asm("prmt.b32 %0, %1, 0, 0xBB99;" : "=r"(pos) : "r"(e));
     neg = ~pos & 0x00010001u;
     return (e ^ (~pos | kBias2)) + neg;
+}
+
+// Deltas that all fit 8 bits (biased by 0x8080) to the planes of their sign-magnitude codes:
+// gathered to bytes, 8x8 blocks transposed, half the work of the 32x32 transpose.  lo, hi: planes
+// 0..7 of the low and high codes (7: magnitude 128), sl, sh: their signs.
+__device__ __forceinline__ void byte_planes(const uint32_t (&w)[32], uint32_t (&lo)[8], uint32_t (&hi)[8], uint32_t& sl,
+                                            uint32_t& sh)
+{
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {  // the low (high) codes of pairs i, 8 + i, 16 + i, 24 + i
+        const uint32_t x = __byte_perm(w[i], w[8 + i], 0x6240), y = __byte_perm(w[16 + i], w[24 + i], 0x6240);
+        lo[i] = __byte_perm(x, y, 0x5410), hi[i] = __byte_perm(x, y, 0x7632);
+    }
+    transpose8(lo);
+    transpose8(hi);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t (&p)[8] = h ? hi : lo;
+        const uint32_t s = ~p[7];
+        uint32_t       c = s;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            const uint32_t b = p[i];
+            p[i]             = b ^ s ^ c;
+            c                = (b ^ s) & c;
+        }
+        p[7] = c;
+        (h ? sh : sl) = s;
+    }
 }
 
 // Bit k of v to bit 2 k (k < 16).

@@ -50,6 +50,20 @@ def test_staged_streams(fz, oracle, ws, dims, extra):
         check(fz, oracle, ws, data, dims, 0.5 / float(data.max() - data.min()), True, 1)
 
 
+@pytest.mark.parametrize("dims", [(900, 70, 1), (4101, 11, 1), (70, 30, 21), (501, 37, 17)],
+                         ids=["2d", "2d-wide", "3d", "3d-odd"])
+@pytest.mark.parametrize("top", [15, 16, 17, 31, 32, 33])
+def test_staged_byte_deltas(fz, oracle, ws, dims, top):
+    """Deltas around the 8 bits below which a block's planes 8..14 are left out: values of +-top
+    give sums of four (2D) and eight (3D) of up to 128 either way, -128 among them."""
+    n = dims[0] * dims[1] * dims[2]
+    rng = np.random.default_rng(top)
+    data = (top * rng.choice([-1, 1], n)).astype(np.float32)
+    data[n // 2:] = (data[n // 2:] * rng.integers(0, 2, n - n // 2)).astype(np.float32)
+    for mode in (0, 1):
+        check(fz, oracle, ws, data, dims, 0.5, False, mode)
+
+
 @pytest.mark.parametrize("dims", [(40000, 1, 1), (400, 101, 1), (4101, 11, 1), (70, 30, 21)],
                          ids=["1d", "2d", "2d-wide", "3d"])
 def test_staged_bounds(fz, oracle, ws, dims):
