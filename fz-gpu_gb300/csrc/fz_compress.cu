@@ -1131,7 +1131,7 @@ __device__ __forceinline__ void range_items(const float* __restrict__ in, uint32
     }
     if ((uint64_t)(i + cnt) * kRangeItemElems >= n && tid < n - 4 * n4) {
         const float x = in[4 * n4 + tid];
-        mn = fminf(mn, x), mx = fmaxf(mx, x);
+        mn = fmin_nan(mn, x), mx = fmax_nan(mx, x);  // (a NaN of the loads above stays)
         nonfinite |= !isfinite(x);
     }
 }

@@ -80,3 +80,16 @@ def test_staged_bounds(fz, oracle, ws, dims):
     data = base.copy()
     data[n // 3] = np.nan
     check(fz, oracle, ws, data, dims, 0.5, False, 1)
+
+
+@pytest.mark.parametrize("n", [5001, 16387, 40001, (1 << 22) + 3])
+def test_nan_before_the_last_elements(fz, ws, n):
+    """A NaN in the elements that the threads holding the last n mod 4 elements read before them."""
+    w = ws if n <= 1 << 20 else fz.Workspace(n)
+    last = (n - 1) // 1024 * 1024
+    for pos in {0, 1, last, max(0, last - 1024), max(0, last - 3 * 1024 + 4), last // 16384 * 16384}:
+        x = np.linspace(0, 1, n, dtype=np.float32)
+        x[pos] = np.nan
+        with pytest.raises(fz.FzError) as e:
+            fz.compress(torch.from_numpy(x).cuda(), (n, 1, 1), 1e-3, rel=True, ws=w)
+        assert e.value.status == fz.NONFINITE_INPUT, pos
