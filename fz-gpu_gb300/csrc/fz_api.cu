@@ -381,6 +381,22 @@ static fz_status compress_args(const float* d_in, uint64_t n, fz_dims dims, doub
     return FZ_SUCCESS;
 }
 
+// The size and status of the stream whose header and status word the last launch left in the
+// pinned mirror, or in `mirror` (syncs).
+static fz_status read_size(fz_workspace* ws, const Layout& L, const uint32_t* mirror, uint64_t* out_bytes, cudaStream_t s)
+{
+    *out_bytes    = L.off_b;
+    cudaError_t e = mirror ? cudaMemcpyAsync(ws->h_pinned, mirror, 68, cudaMemcpyDeviceToHost, s) : cudaSuccess;
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
+    fz_header h;
+    uint32_t  bits;
+    std::memcpy(&h, ws->h_pinned, 64);
+    std::memcpy(&bits, ws->h_pinned + 64, 4);
+    *out_bytes = L.off_b + 16ull * h.nnz;
+    return take_status(ws, bits, s);
+}
+
 // fz_compress with an optional device mirror of the header and status word (128 bytes,
 // written by the last kernel; the request loop reads both with one copy).
 fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_dims dims, double eb,
@@ -416,6 +432,13 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     J.s2off   = group_sum_l2(ws->max_tiles);
     J.rel    = eb_mode == FZ_EB_REL;
     field_items(L.n, L.nb, a.ntiles, J.rel != 0, J.nr, J.ne, J.nc);
+    if (J.ne <= kSmallItems) {  // one launch (and the call before leaves its range to it, see below)
+        KernelTimer       t(ws, s, 1);
+        const cudaError_t e = launch_small_field((int)L.ndim, J, s);
+        if (e != cudaSuccess) return map_err(e);
+        if (ra) ra->done = false;
+        return out_bytes ? read_size(ws, L, mirror, out_bytes, s) : FZ_SUCCESS;
+    }
     if (ra && ra->have && J.rel) J.nr = 0;  // the previous call's encode launch took the range
     // range ahead: only when a compaction launch follows the encode launch (it moves the
     // accumulated range into place once every encode CTA has finished)
@@ -425,9 +448,9 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
         CompressArgs    an;
         if (f.n <= ws->max_n && compress_args(static_cast<const float*>(f.src), f.n, f.dims, f.eb, eb_mode, mode, f.dst,
                                               f.dst_capacity, ws->status, Ln, an) == FZ_SUCCESS) {
-            uint32_t ne, nc;
-            field_items(Ln.n, Ln.nb, an.ntiles, true, J.ahead_nr, ne, nc);
-            J.ahead_in = an.in, J.ahead_n = an.n;
+            uint32_t nr, ne, nc;
+            field_items(Ln.n, Ln.nb, an.ntiles, true, nr, ne, nc);
+            if (ne > kSmallItems) J.ahead_nr = nr, J.ahead_in = an.in, J.ahead_n = an.n;
         }
     }
     cudaError_t e = cudaSuccess;
@@ -445,21 +468,7 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     }
     if (e != cudaSuccess) return map_err(e);
     if (ra) ra->done = J.ahead_nr != 0;
-    if (out_bytes) {
-        if (mirror) e = cudaMemcpyAsync(ws->h_pinned, mirror, 68, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            *out_bytes = L.off_b;
-            return map_err(e, FZ_FAIL_GPU_MEMCPY);
-        }
-        fz_header h;
-        uint32_t  bits;
-        std::memcpy(&h, ws->h_pinned, 64);
-        std::memcpy(&bits, ws->h_pinned + 64, 4);
-        *out_bytes = L.off_b + 16ull * h.nnz;
-        return take_status(ws, bits, s);
-    }
-    return FZ_SUCCESS;
+    return out_bytes ? read_size(ws, L, mirror, out_bytes, s) : FZ_SUCCESS;
 }
 
 extern "C" {

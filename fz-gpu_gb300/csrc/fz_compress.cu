@@ -10,6 +10,8 @@
 //   k_compact_fields  the prefix sum over the blocks' chunk counts (replacing
 //                     cub::DeviceScan, fz.cu:187-201) from per-group sums, the move of the
 //                     chunks to their final offsets, the offset table and the header.
+//   k_small_field     the three in one launch of one cluster, for a single field of at most
+//                     kSmallItems encode items.
 //   k_range, k_compress  the same forward path with a decoupled look-back over scan
 //                     tiles in a single persistent launch after a range pass; used where no
 //                     scratch for the slots exists (fz_compress_noalloc).
@@ -22,6 +24,8 @@
 // chunks with 128-bit stores.
 #include <algorithm>
 #include <atomic>
+
+#include <cooperative_groups.h>
 
 #include "fz_encode.cuh"
 #include "fz_internal.h"
@@ -1039,7 +1043,8 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_compress(const Compr
 //                      counts are known: the group sums before it plus the counts in its
 //                      group), the offset table, the chunks moved from the slots to
 //                      Section B; the field's last item writes the header
-// A single field is a list of one whose job is a kernel parameter.  The stream bytes equal
+// A single field is a list of one whose job is a kernel parameter (one of at most kSmallItems
+// encode items goes to k_small_field).  The stream bytes equal
 // the single-pass look-back kernel's.
 constexpr uint32_t kCompactBlocks = 32;   // shuffle blocks per compaction item
 // CTAs per SM the encode kernels are built for: the 3D variants spill at 64 registers (500x500x100
@@ -1142,6 +1147,10 @@ __device__ __forceinline__ void range_items(const float* __restrict__ in, uint32
 // block's count for the compaction launch.
 constexpr uint32_t kCountPar = 1u << 31;
 
+// encode_item's `packed` for a field of known range.
+template <int ND>
+__device__ __forceinline__ uint32_t packed_kind(const EbInfo& eb) { return !packed_range<ND>(eb) ? 0u : eb.vmin >= 0.0f ? 3u : 1u; }
+
 // Block t's non-zero chunks (lane's: lane + 32 k) into its slot, its count into counts[] and
 // the group sums.
 template <bool kBytes = false>
@@ -1167,9 +1176,16 @@ __device__ __forceinline__ void emit_block(const FieldJob& J, uint32_t t, uint32
     }
 }
 
-// Block t of field J in the float path.
-template <int ND>
-__device__ __forceinline__ void float_block(const FieldJob& J, uint32_t t, float r, uint32_t par, uint32_t* sm)
+// What is left of a warp's block once its image is in shared memory: its bitmap words, its chunk
+// count, and whether a code overflowed its field.
+struct BlockCodes {
+    uint32_t bm[8], cnt, ovf;
+};
+
+// Block t of field J in the float path.  kEmit: its chunks go to its slot; otherwise they are left
+// in the image, described by `out`.
+template <int ND, bool kEmit>
+__device__ __forceinline__ void float_block(const FieldJob& J, uint32_t t, float r, uint32_t par, uint32_t* sm, BlockCodes& out)
 {
     const uint32_t      lane = threadIdx.x & 31u;
     const CompressArgs& a    = J.a;
@@ -1179,6 +1195,12 @@ __device__ __forceinline__ void float_block(const FieldJob& J, uint32_t t, float
     uint32_t* signw = (ND == 1 && a.mode == 1) ? reinterpret_cast<uint32_t*>(a.out + a.off_sign) : nullptr;
     uint32_t  bm[8] = {0, 0, 0, 0, 0, 0, 0, 0}, cnt = 0, ovf = 0;
     compute_block<ND>(a, g, t, r, lane, sm, signw, bm, cnt, ovf);  // warp-uniform t
+    if constexpr (!kEmit) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) out.bm[k] = bm[k];
+        out.cnt = cnt, out.ovf = ovf;
+        return;
+    }
     if (t < a.nb) {
         uint4 c[8];
 #pragma unroll
@@ -1223,8 +1245,9 @@ __device__ __noinline__ void packed_tail(const CompressArgs& a, const uint32_t* 
 // Block t of field J from the staged item (fz_encode.cuh), all of it inside x*y*z, or the
 // tail (t == nb).  Holds one CTA barrier: every warp has read the staged values, and the images
 // take their place.
-template <int ND, bool kRow, int kX, bool kNarrow>
-__device__ __forceinline__ void packed_block(const FieldJob& J, uint32_t t, uint32_t halo, uint32_t par, uint32_t* smem)
+template <int ND, bool kRow, int kX, bool kNarrow, bool kEmit>
+__device__ __forceinline__ void packed_block(const FieldJob& J, uint32_t t, uint32_t halo, uint32_t par, uint32_t* smem,
+                                             BlockCodes& out)
 {
     const uint32_t      lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const CompressArgs& a    = J.a;
@@ -1245,7 +1268,13 @@ __device__ __forceinline__ void packed_block(const FieldJob& J, uint32_t t, uint
         for (int p = 0; p < 8; ++p) v[p] = lo[p], v[8 + p] = 0u, v[16 + p] = hi[p], v[24 + p] = 0u;
         v[15] = slow, v[31] = shigh;
         flag_block<true>(a, t, lane, v, sm, bm, cnt, c);
-        emit_block<true>(J, t, lane, c, bm, cnt, par);
+        if constexpr (kEmit) {
+            emit_block<true>(J, t, lane, c, bm, cnt, par);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) out.bm[k] = bm[k];
+            out.cnt = cnt;
+        }
         return;
     }
     if (ND != 1) {
@@ -1266,18 +1295,25 @@ __device__ __forceinline__ void packed_block(const FieldJob& J, uint32_t t, uint
         *reinterpret_cast<uint2*>(a.out + a.off_sign + (size_t)t * (kBlockCodes / 8) + 8 * lane) =
             make_uint2(spread16(slow & 0xFFFFu) | (spread16(shigh & 0xFFFFu) << 1), spread16(slow >> 16) | (spread16(shigh >> 16) << 1));
     flag_block<false>(a, t, lane, w, sm, bm, cnt, c);
-    emit_block(J, t, lane, c, bm, cnt, par);
+    if constexpr (kEmit) {
+        emit_block(J, t, lane, c, bm, cnt, par);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) out.bm[k] = bm[k];
+        out.cnt = cnt;
+    }
 }
 
-// Encode item i of field J.  packed: 1 the field's range is known to fit the 16-bit path, 3 and
+// Item `item` of field J: the warps' blocks (or the tail), their chunks to the slots (kEmit) or
+// left in the images.  packed: 1 the field's range is known to fit the 16-bit path, 3 and
 // no value is negative, 2 to be found per item, 0 neither.
-template <int ND>
-__device__ __forceinline__ void encode_item(const FieldJob& J, uint32_t i, float r, uint32_t par, uint32_t packed,
-                                            uint32_t* smem)
+template <int ND, bool kEmit>
+__device__ __forceinline__ void encode_item(const FieldJob& J, uint32_t item, float r, uint32_t par, uint32_t packed,
+                                            uint32_t* smem, BlockCodes& out)
 {
     const uint32_t      wid  = threadIdx.x >> 5;
     const CompressArgs& a    = J.a;
-    const uint32_t      item = J.ne - 1 - i, base = item * kItemCodes, t = item * kCompressWarps + wid;
+    const uint32_t      base = item * kItemCodes, t = item * kCompressWarps + wid;
     StagePlan           p;
     if (packed && base < a.nl && a.n >= 64 && stage_plan<ND>(a.x, a.xy, a.dx, a.dxy, p)) {
         uint8_t*   stage = reinterpret_cast<uint8_t*>(smem);
@@ -1294,21 +1330,21 @@ __device__ __forceinline__ void encode_item(const FieldJob& J, uint32_t i, float
         if (!__syncthreads_or(track && !(amax < packed_limit<ND>()))) {
             if ((t + 1) * kBlockCodes <= a.nl || (t == a.nb && t * kBlockCodes < a.n)) {
                 const int xm = a.al_x ? 0 : a.x % 2 ? 1 : 2;  // how the row above is read
-                if (ND == 1) packed_block<1, false, 0, false>(J, t, p.halo, par, smem);
-                else if (ND == 2 && p.shift && xm == 0) packed_block<ND, false, 0, false>(J, t, p.halo, par, smem);
-                else if (ND == 2 && p.shift) packed_block<ND, false, 1, false>(J, t, p.halo, par, smem);
-                else if (a.x < 64 && xm == 0) packed_block<ND, true, 0, true>(J, t, p.halo, par, smem);
-                else if (a.x < 64 && xm == 2) packed_block<ND, true, 2, true>(J, t, p.halo, par, smem);
-                else if (a.x < 64) packed_block<ND, true, 1, true>(J, t, p.halo, par, smem);
-                else if (xm == 0) packed_block<ND, true, 0, false>(J, t, p.halo, par, smem);
-                else if (xm == 2) packed_block<ND, true, 2, false>(J, t, p.halo, par, smem);
-                else packed_block<ND, true, 1, false>(J, t, p.halo, par, smem);
+                if (ND == 1) packed_block<1, false, 0, false, kEmit>(J, t, p.halo, par, smem, out);
+                else if (ND == 2 && p.shift && xm == 0) packed_block<ND, false, 0, false, kEmit>(J, t, p.halo, par, smem, out);
+                else if (ND == 2 && p.shift) packed_block<ND, false, 1, false, kEmit>(J, t, p.halo, par, smem, out);
+                else if (a.x < 64 && xm == 0) packed_block<ND, true, 0, true, kEmit>(J, t, p.halo, par, smem, out);
+                else if (a.x < 64 && xm == 2) packed_block<ND, true, 2, true, kEmit>(J, t, p.halo, par, smem, out);
+                else if (a.x < 64) packed_block<ND, true, 1, true, kEmit>(J, t, p.halo, par, smem, out);
+                else if (xm == 0) packed_block<ND, true, 0, false, kEmit>(J, t, p.halo, par, smem, out);
+                else if (xm == 2) packed_block<ND, true, 2, false, kEmit>(J, t, p.halo, par, smem, out);
+                else packed_block<ND, true, 1, false, kEmit>(J, t, p.halo, par, smem, out);
                 return;
             }
             __syncthreads();
         }
     }
-    float_block<ND>(J, t, r, par, smem + wid * kBlockWords);
+    float_block<ND, kEmit>(J, t, r, par, smem + wid * kBlockWords, out);
 }
 
 // The words the header of field J follows from, loaded by the thread that will write it as
@@ -1538,7 +1574,7 @@ __global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas<ND>)
             // the call's group-sum set (the compaction launch moves the counter on)
             if (J.rel) {
                 const EbInfo eb = eb_from_range(ord2f(__ldcg(J.ctl->mm)), ord2f(__ldcg(J.ctl->mm + 1)), J.a.eb_rel);
-                s_r = eb.ebx2_r, s_packed = !packed_range<ND>(eb) ? 0u : eb.vmin >= 0.0f ? 3u : 1u;
+                s_r = eb.ebx2_r, s_packed = packed_kind<ND>(eb);
             } else {
                 s_r = J.a.ebh.ebx2_r, s_packed = 2u;
             }
@@ -1546,7 +1582,10 @@ __global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas<ND>)
             s_rf  = f;
         }
         __syncthreads();
-        encode_item<ND>(J, i, s_r, s_par, s_packed, esm);
+        // the last item first: the range launch read the field front to back, so its end is the part
+        // most likely still in L2
+        BlockCodes unused;
+        encode_item<ND, true>(J, J.ne - 1 - i, s_r, s_par, s_packed, esm, unused);
         __syncthreads();  // the blocks' shared images before the next item
         // a field without full shuffle blocks has one encode item and no compaction: the
         // header is written here (its counter stays, no group sums were used)
@@ -1555,6 +1594,115 @@ __global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas<ND>)
     if constexpr (!kList) {
         if (one.ahead_nr) range_ahead(one, total);
     }
+}
+
+// A whole small field in one launch: a cluster of one CTA per encode item (at most kSmallItems).
+// Each CTA takes the max/min of its item's elements, the cluster's CTAs exchange them through
+// distributed shared memory, each encodes its item, and from the exchanged chunk counts writes its
+// chunks straight to Section B; the last item's CTA writes the header.  No word of the
+// workspace but the status is used.  A field this small is bound by latencies: three launches,
+// each followed by the first loads of the next, the chunks' way through their slots, the group sums.
+// fz_compress on GB300, relative bound 1e-3, three launches -> this kernel, called with the size
+// read back / in a graph: 128x128 36.8 -> 29.9 / 12.3 -> 6.8 us, 362x362 (unaligned rows) 38.9 ->
+// 33.8 / 14.2 -> 10.3, 512x512 37.0 -> 32.4 / 13.2 -> 9.0, 64x64x64 35.9 -> 32.8 / 12.7 -> 9.5;
+// in the float path (1e-5) 512x512 41.2 -> 34.3 / 17.3 -> 11.0.
+template <int ND>
+__global__ void __launch_bounds__(kCompressWarps * 32, 3) k_small_field(const __grid_constant__ FieldJob J)
+{
+    namespace cg = cooperative_groups;
+    pdl_wait();
+    pdl_trigger();
+    extern __shared__ __align__(16) uint32_t esm[];
+    __shared__ uint32_t s_red[3][kCompressWarps], s_mine[3];  // min, max as ordered u32, non-finite; then counts
+    __shared__ uint32_t s_cnt[kCompressWarps], s_ovf[kCompressWarps], s_pre[kCompressWarps], s_tot[2], s_packed, s_bad;
+    __shared__ EbInfo   s_eb;
+    cg::cluster_group   cluster = cg::this_cluster();
+    const CompressArgs& a    = J.a;
+    const uint32_t      tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
+    const uint32_t      item = blockIdx.x, items = gridDim.x;
+    if (J.rel) {
+        // this item's elements, 16 range items of 1024
+        const uint32_t r0 = item * (kItemCodes / kRangeItemElems), r1 = min(r0 + kItemCodes / kRangeItemElems, (uint32_t)cdiv(a.n, kRangeItemElems));
+        float          mn = INFINITY, mx = -INFINITY;
+        uint32_t       nonfinite = 0;
+        for (uint32_t r = r0; r < r1; r += kRangeBatch) range_items(a.in, a.n, r, min(kRangeBatch, r1 - r), mn, mx, nonfinite);
+        nonfinite |= (mn != mn) | (mn == -INFINITY) | (mx == INFINITY);  // (as in range_flush)
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
+            mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+        }
+        nonfinite = __reduce_or_sync(kFull, nonfinite);
+        if (lane == 0) s_red[0][wid] = f2ord(mn), s_red[1][wid] = f2ord(mx), s_red[2][wid] = nonfinite;
+        __syncthreads();
+        if (wid == 0) {
+            const uint32_t lo = __reduce_min_sync(kFull, lane < kCompressWarps ? s_red[0][lane] : 0xFFFFFFFFu);
+            const uint32_t hi = __reduce_max_sync(kFull, lane < kCompressWarps ? s_red[1][lane] : 0u);
+            const uint32_t nf = __reduce_or_sync(kFull, lane < kCompressWarps ? s_red[2][lane] : 0u);
+            if (lane == 0) s_mine[0] = lo, s_mine[1] = hi, s_mine[2] = nf;
+        }
+        cluster.sync();
+        if (wid == 0) {
+            const uint32_t* peer = lane < items ? cluster.map_shared_rank(s_mine, lane) : nullptr;
+            const uint32_t  lo   = __reduce_min_sync(kFull, peer ? peer[0] : 0xFFFFFFFFu);
+            const uint32_t  hi   = __reduce_max_sync(kFull, peer ? peer[1] : 0u);
+            const uint32_t  nf   = __reduce_or_sync(kFull, peer ? peer[2] : 0u);
+            if (lane == 0) {
+                s_eb     = eb_from_range(ord2f(lo), ord2f(hi), a.eb_rel);
+                s_packed = packed_kind<ND>(s_eb), s_bad = nf ? 1u : 0u;
+            }
+        }
+    } else if (tid == 0) {
+        s_eb = a.ebh, s_packed = 2u, s_bad = 0u;
+    }
+    __syncthreads();
+    BlockCodes c{};
+    encode_item<ND, false>(J, item, s_eb.ebx2_r, 0u, s_packed, esm, c);
+    if (lane == 0) s_cnt[wid] = c.cnt, s_ovf[wid] = c.ovf;
+    __syncthreads();
+    if (wid == 0) {
+        const uint32_t n   = lane < kCompressWarps ? s_cnt[lane] : 0u;
+        const uint32_t tot = __reduce_add_sync(kFull, n), ovf = __reduce_or_sync(kFull, lane < kCompressWarps ? s_ovf[lane] : 0u);
+        uint32_t       inc = n;
+#pragma unroll
+        for (uint32_t o = 1; o < kCompressWarps; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(kFull, inc, o);
+            if (lane >= o) inc += v;
+        }
+        if (lane < kCompressWarps) s_pre[lane] = inc - n;
+        if (lane == 0) s_tot[0] = tot, s_tot[1] = ovf;
+    }
+    cluster.sync();
+    const uint32_t  t = item * kCompressWarps + wid;
+    const uint32_t* peer = lane < items ? cluster.map_shared_rank(s_tot, lane) : nullptr;
+    const uint32_t  pt = peer ? peer[0] : 0u;
+    const uint32_t  excl = __reduce_add_sync(kFull, lane < item ? pt : 0u);
+    if (t < a.nb) {
+        uint32_t        pre = excl + s_pre[wid];
+        const uint32_t* sm  = esm + wid * kBlockWords;
+        uint4*          B   = reinterpret_cast<uint4*>(a.out + a.off_b);
+        const uint32_t  lt  = lanemask_lt();
+        if (a.boff && lane == 0) a.boff[t] = pre;
+#pragma unroll
+        for (uint32_t u = 0; u < 8; ++u) {
+            if ((c.bm[u] >> lane) & 1u)
+                B[pre + __popc(c.bm[u] & lt)] = *reinterpret_cast<const uint4*>(sm + (lane + 32 * u) * 4);
+            pre += __popc(c.bm[u]);
+        }
+    }
+    if (item == items - 1 && wid == 0) {
+        const uint32_t total = __reduce_add_sync(kFull, pt), ovf = __reduce_or_sync(kFull, peer ? peer[1] : 0u);
+        if (lane == 0) {
+            const uint32_t st = s_bad ? atomicOr(a.status, kStatusNonfinite) | kStatusNonfinite : a.mirror ? __ldcg(a.status) : 0u;
+            write_header(a, s_eb, (ovf ? 1u : 0u) | (s_bad ? 2u : 0u), total, reinterpret_cast<uint4*>(a.mirror));
+            if (a.mirror) a.mirror[16] = st;
+            if (a.boff) {
+                a.boff[a.nb] = total;  // the total closes the offset table; zero its 16-byte pad
+                for (uint32_t k = a.nb + 1; k < (uint32_t)(pad16(4ull * (a.nb + 1)) / 4); ++k) a.boff[k] = 0;
+            }
+        }
+    }
+    cluster.sync();  // no CTA leaves while another reads its counts
 }
 
 template <bool kList>
@@ -1678,6 +1826,35 @@ cudaError_t launch_fields(FieldPhase phase, int nd, const FieldJob* jobs, const 
     case 1: return launch_pdl(k_encode_fields<1, false>, grid, block, encode_smem<1>(), s, jobs, segs, nseg, total, one);
     case 2: return launch_pdl(k_encode_fields<2, false>, grid, block, encode_smem<2>(), s, jobs, segs, nseg, total, one);
     default: return launch_pdl(k_encode_fields<3, false>, grid, block, encode_smem<3>(), s, jobs, segs, nseg, total, one);
+    }
+}
+
+// k_small_field<ND> opted in to its dynamic shared memory and clusters past 8 CTAs on the current
+// device.
+template <int ND>
+static cudaError_t allow_small()
+{
+    static std::atomic<uint64_t> done{0};  // bit d: opted in on device d
+    int         dev = 0;
+    cudaError_t e   = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
+    if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+    e = cudaFuncSetAttribute(k_small_field<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)encode_smem<ND>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_field<ND>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+}
+
+cudaError_t launch_small_field(int nd, const FieldJob& J, cudaStream_t s)
+{
+    const cudaError_t e = nd == 1 ? allow_small<1>() : nd == 2 ? allow_small<2>() : allow_small<3>();
+    if (e != cudaSuccess) return e;
+    const dim3 grid(J.ne), block(kCompressWarps * 32);
+    switch (nd) {
+    case 1: return launch_pdl_cluster(k_small_field<1>, grid, block, encode_smem<1>(), s, J.ne, J);
+    case 2: return launch_pdl_cluster(k_small_field<2>, grid, block, encode_smem<2>(), s, J.ne, J);
+    default: return launch_pdl_cluster(k_small_field<3>, grid, block, encode_smem<3>(), s, J.ne, J);
     }
 }
 

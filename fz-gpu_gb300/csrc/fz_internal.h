@@ -117,23 +117,43 @@ __host__ __device__ inline uint32_t group_sum_words(uint32_t nb) { return group_
 // eager launches on one stream 2043 -> 2210 GB/s; in graphs, which already have no launch
 // gaps, 1 branch unchanged, 16 branches -1.2% and list launches -3% (the early CTAs wait on
 // SMs that other branches' kernels would use), so captured launches go without it.
+// cluster: CTAs per cluster (a divisor of the grid), 1 for none.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                              const Args&... args)
+inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                      uint32_t cluster, const Args&... args)
 {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
         (void)cudaGetLastError();  // a query that failed leaves no error behind
         cs = cudaStreamCaptureStatusActive;
     }
-    cudaLaunchAttribute at{};
-    at.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2]{};
+    uint32_t            na = 0;
+    if (cs == cudaStreamCaptureStatusNone) {
+        at[na].id                                           = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[na].id               = cudaLaunchAttributeClusterDimension;
+        at[na++].val.clusterDim = {cluster, 1, 1};
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = s;
-    cfg.attrs = &at, cfg.numAttrs = cs == cudaStreamCaptureStatusNone ? 1u : 0u;
+    cfg.attrs = at, cfg.numAttrs = na;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                              const Args&... args)
+{
+    return launch_pdl_cluster(kernel, grid, block, smem, s, 1u, args...);
+}
+
+// Single fields of at most this many encode items (16384 codes each) are compressed by one launch of
+// one cluster: the largest cluster there is, and at 16 items the launch still takes less time than
+// the three (figures at k_small_field).
+constexpr uint32_t kSmallItems = 16;
+cudaError_t launch_small_field(int nd, const FieldJob& J, cudaStream_t s);
 
 // Items of each kind for a field of n elements (ntiles scan tiles of shuffle blocks, nb full
 // blocks).
