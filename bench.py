@@ -357,7 +357,7 @@ def run_fz(args, rank, world, local_rank):
     torch.cuda.synchronize()
     kern = {k: ws.kernel_time(k) for k in fz.Workspace.KERNELS}
     ws.enable_timing(0)
-    launches = args.steps * sum(c for c, _ in kern.values()) // ksteps  # region 1 launches the same kernels
+    launches = args.steps * sum(c for c, _ in kern.values()) // ksteps  # region 1 launches the same kernels (or more: small fields)
     # Timed region 3 (value_without_graphs): the same steps as one batch call per direction
     # on one stream, without graphs (each field's encode launch also takes the next field's
     # range there), CUDA events around the whole region only.
@@ -462,9 +462,11 @@ def kernel_table(kern, n, stream_b, dims, hbm):
             "k_compact_fields": 2 * stream_b + 8 * (nb + 1), "k_offsets": 4 * ((n + 255) // 256) + 4 * (nb + 1),
             "k_decompress": stream_b + 4 * n, "k_recon": 2 * n + 4 * n}
     nd = 3 if dims[2] > 1 else (2 if dims[1] > 1 else 1)
-    # the names ncu shows: the encode kernel is templated on the dimensionality, the fused
-    # decompression kernel has one variant per dimensionality and a second 2D one
-    shown = {"k_encode_fields": f"k_encode_fields<{nd}>", "k_decompress": decompress_kernel(dims)}
+    # the names ncu shows: the encode kernel is templated on the dimensionality (a field of at most
+    # one wave of CTAs, compressed by one call, has no compaction launch), the fused decompression
+    # kernel has one variant per dimensionality
+    encode = "k_encode_fields" if kern["k_compact_fields"][0] else "k_whole_field"
+    shown = {"k_encode_fields": f"{encode}<{nd}>", "k_decompress": decompress_kernel(dims)}
     total = sum(v[1] for v in kern.values()) or 1.0
     kernels = {}
     for k, (cnt, tot) in kern.items():

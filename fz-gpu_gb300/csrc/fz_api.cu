@@ -432,17 +432,11 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     J.s2off   = group_sum_l2(ws->max_tiles);
     J.rel    = eb_mode == FZ_EB_REL;
     field_items(L.n, L.nb, a.ntiles, J.rel != 0, J.nr, J.ne, J.nc);
-    if (J.ne <= kSmallItems) {  // one launch (and the call before leaves its range to it, see below)
-        KernelTimer       t(ws, s, 1);
-        const cudaError_t e = launch_small_field((int)L.ndim, J, s);
-        if (e != cudaSuccess) return map_err(e);
-        if (ra) ra->done = false;
-        return out_bytes ? read_size(ws, L, mirror, out_bytes, s) : FZ_SUCCESS;
-    }
-    if (ra && ra->have && J.rel) J.nr = 0;  // the previous call's encode launch took the range
+    const bool small = J.ne <= kSmallItems, whole = small || (!ra && whole_field_fits((int)L.ndim, J.ne));
+    if (small || (ra && ra->have && J.rel)) J.nr = 0;  // the launch itself, or the previous call's encode launch, takes the range
     // range ahead: only when a compaction launch follows the encode launch (it moves the
     // accumulated range into place once every encode CTA has finished)
-    if (ra && ra->next && J.rel && J.nc) {
+    if (ra && ra->next && J.rel && J.nc && !whole) {
         const fz_field& f = *ra->next;
         Layout          Ln;
         CompressArgs    an;
@@ -460,9 +454,10 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     }
     if (e == cudaSuccess) {
         KernelTimer t(ws, s, 1);
-        e = launch_fields(FieldPhase::Encode, (int)L.ndim, nullptr, nullptr, 0, J.ne, J, s, J.ahead_nr);
+        e = whole ? launch_whole_field((int)L.ndim, J, s)
+                  : launch_fields(FieldPhase::Encode, (int)L.ndim, nullptr, nullptr, 0, J.ne, J, s, J.ahead_nr);
     }
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && !whole) {
         KernelTimer t(ws, s, 5);
         e = launch_fields(FieldPhase::Compact, (int)L.ndim, nullptr, nullptr, 0, J.nc, J, s);
     }

@@ -10,8 +10,9 @@
 //   k_compact_fields  the prefix sum over the blocks' chunk counts (replacing
 //                     cub::DeviceScan, fz.cu:187-201) from per-group sums, the move of the
 //                     chunks to their final offsets, the offset table and the header.
-//   k_small_field     the three in one launch of one cluster, for a single field of at most
-//                     kSmallItems encode items.
+//   k_whole_field     the three in one launch for a single field: of one cluster, range
+//                     included, up to kSmallItems encode items; after a range launch, up to
+//                     one resident wave of items.
 //   k_range, k_compress  the same forward path with a decoupled look-back over scan
 //                     tiles in a single persistent launch after a range pass; used where no
 //                     scratch for the slots exists (fz_compress_noalloc).
@@ -1043,8 +1044,8 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_compress(const Compr
 //                      counts are known: the group sums before it plus the counts in its
 //                      group), the offset table, the chunks moved from the slots to
 //                      Section B; the field's last item writes the header
-// A single field is a list of one whose job is a kernel parameter (one of at most kSmallItems
-// encode items goes to k_small_field).  The stream bytes equal
+// A single field is a list of one whose job is a kernel parameter (one of at most
+// a resident wave of encode items goes to k_whole_field).  The stream bytes equal
 // the single-pass look-back kernel's.
 constexpr uint32_t kCompactBlocks = 32;   // shuffle blocks per compaction item
 // CTAs per SM the encode kernels are built for: the 3D variants spill at 64 registers (500x500x100
@@ -1596,31 +1597,55 @@ __global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas<ND>)
     }
 }
 
-// A whole small field in one launch: a cluster of one CTA per encode item (at most kSmallItems).
-// Each CTA takes the max/min of its item's elements, the cluster's CTAs exchange them through
-// distributed shared memory, each encodes its item, and from the exchanged chunk counts writes its
-// chunks straight to Section B; the last item's CTA writes the header.  No word of the
-// workspace but the status is used.  A field this small is bound by latencies: three launches,
-// each followed by the first loads of the next, the chunks' way through their slots, the group sums.
-// fz_compress on GB300, relative bound 1e-3, three launches -> this kernel, called with the size
-// read back / in a graph: 128x128 36.8 -> 29.9 / 12.3 -> 6.8 us, 362x362 (unaligned rows) 38.9 ->
-// 33.8 / 14.2 -> 10.3, 512x512 37.0 -> 32.4 / 13.2 -> 9.0, 64x64x64 35.9 -> 32.8 / 12.7 -> 9.5;
-// in the float path (1e-5) 512x512 41.2 -> 34.3 / 17.3 -> 11.0.
-template <int ND>
-__global__ void __launch_bounds__(kCompressWarps * 32, 3) k_small_field(const __grid_constant__ FieldJob J)
+// A whole field in one launch of one CTA per encode item; the chunks go from the images straight to
+// Section B, with no slots, group sums or compaction launch; the last item's CTA writes the header.
+//
+// kScan false, at most kSmallItems items: the CTAs are one cluster.  Each takes the max/min of its
+// item's elements, they exchange them through distributed shared memory, each encodes its item, and
+// they exchange the chunk counts.  No word of the workspace but the status is used.  A field this
+// small is bound by latencies: three launches, each followed by the first loads of the next, the
+// chunks' way through their slots, the group sums.  fz_compress on GB300, relative bound 1e-3, three
+// launches -> this kernel, called with the size read back / in a graph: 128x128 36.8 -> 29.9 / 12.3
+// -> 6.8 us, 362x362 (unaligned rows) 38.9 -> 33.8 / 14.2 -> 10.3, 512x512 37.0 -> 32.4 / 13.2 -> 9.0,
+// 64x64x64 35.9 -> 32.8 / 12.7 -> 9.5; in the float path (1e-5) 512x512 41.2 -> 34.3 / 17.3 -> 11.0.
+//
+// kScan true, after the range launch, at most one resident wave of items: items are handed out by
+// tickets, each CTA publishes its chunk count and sums the counts of all items before its own (their
+// CTAs have started, and wait for none after them).  Past one wave this loses: CTAs that wait hold
+// the memory the next items need, and all wait for the slowest (a persistent form of it took 43.7 us
+// for the 928 items of 39200x388, the encode and compaction launches 23.5 and 8).  Two launches ->
+// this one, same measures: 1000x1000 38.8 -> 35.3 / 13.6 -> 11.5, 3600x1800 47.4 -> 42.9 / 21.4 ->
+// 20.2, 128x128x128 40.2 -> 38.4 / 15.1 -> 13.2, 4000000 42.2 -> 40.8 / 16.6 -> 15.3; worst 2000x1500
+// 42.7 -> 40.9 / 15.9 -> 16.0 (184 items: 32 of the 152 SMs have two).  A polling thread per count
+// instead of one polling warp: 4000000 in a graph 18.5.  A cooperative launch with the range inside,
+// behind a grid barrier, was no faster than the range launch and cannot overlap its neighbours.
+template <int ND, bool kScan>
+__global__ void __launch_bounds__(kCompressWarps * 32, 3) k_whole_field(const __grid_constant__ FieldJob J)
 {
     namespace cg = cooperative_groups;
     pdl_wait();
     pdl_trigger();
     extern __shared__ __align__(16) uint32_t esm[];
-    __shared__ uint32_t s_red[3][kCompressWarps], s_mine[3];  // min, max as ordered u32, non-finite; then counts
+    __shared__ uint32_t s_red[3][kCompressWarps], s_mine[3];  // min, max as ordered u32, non-finite
     __shared__ uint32_t s_cnt[kCompressWarps], s_ovf[kCompressWarps], s_pre[kCompressWarps], s_tot[2], s_packed, s_bad;
+    __shared__ uint32_t s_item, s_epoch, s_excl, s_prior, s_ok;
     __shared__ EbInfo   s_eb;
     cg::cluster_group   cluster = cg::this_cluster();
     const CompressArgs& a    = J.a;
     const uint32_t      tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
-    const uint32_t      item = blockIdx.x, items = gridDim.x;
-    if (J.rel) {
+    const uint32_t      items = gridDim.x;
+    uint32_t            item  = blockIdx.x;
+    if constexpr (kScan) {
+        if (tid == 0) {
+            s_epoch = __ldcg(a.epoch);
+            __threadfence();  // read before the first ticket (the last one advances it)
+            s_item   = take_ticket(a.ticket, a.epoch, items).tile;
+            s_eb     = J.rel ? eb_from_range(ord2f(__ldcg(J.ctl->mm)), ord2f(__ldcg(J.ctl->mm + 1)), a.eb_rel) : a.ebh;
+            s_packed = J.rel ? packed_kind<ND>(s_eb) : 2u;
+        }
+        __syncthreads();
+        item = s_item;
+    } else if (J.rel) {
         // this item's elements, 16 range items of 1024
         const uint32_t r0 = item * (kItemCodes / kRangeItemElems), r1 = min(r0 + kItemCodes / kRangeItemElems, (uint32_t)cdiv(a.n, kRangeItemElems));
         float          mn = INFINITY, mx = -INFINITY;
@@ -1670,14 +1695,52 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_small_field(const __
             if (lane >= o) inc += v;
         }
         if (lane < kCompressWarps) s_pre[lane] = inc - n;
-        if (lane == 0) s_tot[0] = tot, s_tot[1] = ovf;
+        if (lane == 0) {
+            s_tot[0] = tot, s_tot[1] = ovf;
+            if (kScan) publish(a.state, item, s_epoch, kFlagAgg, ovf ? 1u : 0u, tot);
+        }
     }
-    cluster.sync();
-    const uint32_t  t = item * kCompressWarps + wid;
-    const uint32_t* peer = lane < items ? cluster.map_shared_rank(s_tot, lane) : nullptr;
-    const uint32_t  pt = peer ? peer[0] : 0u;
-    const uint32_t  excl = __reduce_add_sync(kFull, lane < item ? pt : 0u);
-    if (t < a.nb) {
+    uint32_t        excl, prior = 0, pt = 0;
+    const uint32_t* peer = nullptr;
+    bool            ok   = true;
+    if constexpr (kScan) {
+        // the counts of all items before this one: their CTAs took their tickets earlier and wait for
+        // no later one.  One warp polls, four loads a lane in flight.
+        if (wid == 0) {
+            uint32_t v, o, spins = 0;
+            bool     all;
+            do {
+                v = o = 0, all = true;
+                for (uint32_t k0 = 0; k0 < item; k0 += 128) {
+                    uint64_t w[4];
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; ++u) {
+                        const uint32_t k = k0 + 32 * u + lane;
+                        w[u]             = k < item ? ld_state(a.state + k) : state_pack(s_epoch, kFlagAgg, 0, 0);
+                    }
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; ++u) {
+                        all = all && (uint32_t)(w[u] >> 32) == s_epoch && state_flag(w[u]) != 0;
+                        v += state_value(w[u]), o |= state_ovf(w[u]);
+                    }
+                }
+                all = __all_sync(kFull, all);
+                if (!all) __nanosleep(40);  // (polls of many CTAs hold up the counts' way through the L2)
+            } while (!all && ++spins <= kSpinLimit / 16);  // (a round polls up to 20 words a lane)
+            v = __reduce_add_sync(kFull, v), o = __reduce_or_sync(kFull, o);
+            if (lane == 0) s_excl = v, s_prior = o, s_ok = all;
+        }
+        __syncthreads();
+        excl = s_excl, prior = s_prior, ok = s_ok != 0;
+        if (!ok && tid == 0) atomicOr(a.status, kStatusTimeout);
+    } else {
+        cluster.sync();
+        peer = lane < items ? cluster.map_shared_rank(s_tot, lane) : nullptr;
+        pt   = peer ? peer[0] : 0u;
+        excl = __reduce_add_sync(kFull, lane < item ? pt : 0u);
+    }
+    const uint32_t t = item * kCompressWarps + wid;
+    if (ok && t < a.nb) {
         uint32_t        pre = excl + s_pre[wid];
         const uint32_t* sm  = esm + wid * kBlockWords;
         uint4*          B   = reinterpret_cast<uint4*>(a.out + a.off_b);
@@ -1691,18 +1754,27 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_small_field(const __
         }
     }
     if (item == items - 1 && wid == 0) {
-        const uint32_t total = __reduce_add_sync(kFull, pt), ovf = __reduce_or_sync(kFull, peer ? peer[1] : 0u);
-        if (lane == 0) {
-            const uint32_t st = s_bad ? atomicOr(a.status, kStatusNonfinite) | kStatusNonfinite : a.mirror ? __ldcg(a.status) : 0u;
-            write_header(a, s_eb, (ovf ? 1u : 0u) | (s_bad ? 2u : 0u), total, reinterpret_cast<uint4*>(a.mirror));
-            if (a.mirror) a.mirror[16] = st;
-            if (a.boff) {
-                a.boff[a.nb] = total;  // the total closes the offset table; zero its 16-byte pad
-                for (uint32_t k = a.nb + 1; k < (uint32_t)(pad16(4ull * (a.nb + 1)) / 4); ++k) a.boff[k] = 0;
+        if constexpr (kScan) {
+            if (lane == 0) {
+                FieldFinal fin = final_loads(J);
+                if (prior | s_tot[1]) fin.flags |= kCtlOverflow;
+                if (!ok) fin.flags |= kStatusNonfinite, fin.status |= kStatusTimeout;  // marks the stream failed
+                finish_field(J, excl + s_tot[0], fin);
+            }
+        } else {
+            const uint32_t total = __reduce_add_sync(kFull, pt), ovf = __reduce_or_sync(kFull, peer ? peer[1] : 0u);
+            if (lane == 0) {
+                const uint32_t st = s_bad ? atomicOr(a.status, kStatusNonfinite) | kStatusNonfinite : a.mirror ? __ldcg(a.status) : 0u;
+                write_header(a, s_eb, (ovf ? 1u : 0u) | (s_bad ? 2u : 0u), total, reinterpret_cast<uint4*>(a.mirror));
+                if (a.mirror) a.mirror[16] = st;
+                if (a.boff) {
+                    a.boff[a.nb] = total;  // the total closes the offset table; zero its 16-byte pad
+                    for (uint32_t k = a.nb + 1; k < (uint32_t)(pad16(4ull * (a.nb + 1)) / 4); ++k) a.boff[k] = 0;
+                }
             }
         }
     }
-    cluster.sync();  // no CTA leaves while another reads its counts
+    if (!kScan) cluster.sync();  // no CTA leaves while another reads its counts
 }
 
 template <bool kList>
@@ -1829,33 +1901,41 @@ cudaError_t launch_fields(FieldPhase phase, int nd, const FieldJob* jobs, const 
     }
 }
 
-// k_small_field<ND> opted in to its dynamic shared memory and clusters past 8 CTAs on the current
-// device.
-template <int ND>
-static cudaError_t allow_small()
+// CTAs of one resident wave of k_whole_field<ND, kScan> on the current device (0: error), opted in to
+// its dynamic shared memory and to clusters past 8 CTAs.
+template <int ND, bool kScan>
+static uint32_t whole_wave()
 {
-    static std::atomic<uint64_t> done{0};  // bit d: opted in on device d
-    int         dev = 0;
-    cudaError_t e   = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
-    if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_small_field<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)encode_smem<ND>());
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_small_field<ND>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
-    return e;
+    static std::atomic<uint32_t> waves[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::atomic<uint32_t>* slot = dev < 64 ? &waves[dev] : nullptr;
+    uint32_t               w    = slot ? slot->load(std::memory_order_acquire) : 0;
+    if (w) return w;
+    if (!kScan && cudaFuncSetAttribute(k_whole_field<ND, kScan>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        return 0;
+    w = resident_ctas(k_whole_field<ND, kScan>, kCompressWarps * 32, encode_smem<ND>());
+    if (slot) slot->store(w, std::memory_order_release);
+    return w;
 }
 
-cudaError_t launch_small_field(int nd, const FieldJob& J, cudaStream_t s)
+bool whole_field_fits(int nd, uint32_t ne)
 {
-    const cudaError_t e = nd == 1 ? allow_small<1>() : nd == 2 ? allow_small<2>() : allow_small<3>();
-    if (e != cudaSuccess) return e;
+    return ne <= (nd == 1 ? whole_wave<1, true>() : nd == 2 ? whole_wave<2, true>() : whole_wave<3, true>());
+}
+
+template <int ND>
+static cudaError_t launch_whole(const FieldJob& J, cudaStream_t s)
+{
     const dim3 grid(J.ne), block(kCompressWarps * 32);
-    switch (nd) {
-    case 1: return launch_pdl_cluster(k_small_field<1>, grid, block, encode_smem<1>(), s, J.ne, J);
-    case 2: return launch_pdl_cluster(k_small_field<2>, grid, block, encode_smem<2>(), s, J.ne, J);
-    default: return launch_pdl_cluster(k_small_field<3>, grid, block, encode_smem<3>(), s, J.ne, J);
-    }
+    if (J.ne > kSmallItems) return launch_pdl(k_whole_field<ND, true>, grid, block, encode_smem<ND>(), s, J);
+    if (!whole_wave<ND, false>()) return cudaErrorInvalidDevice;
+    return launch_pdl_cluster(k_whole_field<ND, false>, grid, block, encode_smem<ND>(), s, J.ne, J);
+}
+
+cudaError_t launch_whole_field(int nd, const FieldJob& J, cudaStream_t s)
+{
+    return nd == 1 ? launch_whole<1>(J, s) : nd == 2 ? launch_whole<2>(J, s) : launch_whole<3>(J, s);
 }
 
 // One resident wave of k_compress<ND> on the current device.  The 64 KiB of dynamic shared

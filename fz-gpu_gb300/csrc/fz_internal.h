@@ -62,7 +62,7 @@ struct CompressArgs {
 // header).  One field is a list of one, passed as a kernel parameter.
 
 // Per-field control words (device, 32 bytes).  Between calls: mm = pre = {0xFFFFFFFF, 0},
-// flags = pre_flags = 0, and epoch = the number of calls that had full shuffle blocks.
+// flags = pre_flags = 0, and epoch = the number of calls that had a compaction launch.
 // Whoever writes a call's header moves pre/pre_flags into mm/flags and resets pre: a
 // call's encode launch may accumulate the range of the next field compressed with the
 // same control words into pre (range ahead), which that field's encode then reads from mm.
@@ -151,9 +151,11 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 
 // Single fields of at most this many encode items (16384 codes each) are compressed by one launch of
 // one cluster: the largest cluster there is, and at 16 items the launch still takes less time than
-// the three (figures at k_small_field).
+// the three (figures at k_whole_field).  whole_field_fits: `ne` items are one resident wave of the
+// launch that follows a range launch.
 constexpr uint32_t kSmallItems = 16;
-cudaError_t launch_small_field(int nd, const FieldJob& J, cudaStream_t s);
+bool        whole_field_fits(int nd, uint32_t ne);
+cudaError_t launch_whole_field(int nd, const FieldJob& J, cudaStream_t s);
 
 // Items of each kind for a field of n elements (ntiles scan tiles of shuffle blocks, nb full
 // blocks).

@@ -154,8 +154,8 @@ fz_status fz_workspace_status(fz_workspace* ws, fz_stream_t stream);
    pair of CUDA events on the call's stream.  capacity 0 disables it. */
 fz_status fz_workspace_enable_timing(fz_workspace* ws, uint32_t capacity);
 /* Number of recorded launches of one kernel kind (0 range pass, 1 encode -- codes,
-   bitshuffle, flags and per-block compaction into slots; for a field of up to 262144
-   codes the whole compression --, 2 block offsets, 3 decode --
+   bitshuffle, flags and per-block compaction into slots; for a field compressed by one
+   call that fits one wave of CTAs the compaction too, and up to 262144 codes the range --, 2 block offsets, 3 decode --
    fused with the inverse Lorenzo --, 4 separate inverse Lorenzo, 5 compaction -- offsets
    and the move into the stream) and their summed duration; syncs on the last recorded
    event and frees those records. */

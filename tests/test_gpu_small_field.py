@@ -1,7 +1,8 @@
-"""The one-launch compression of small fields (k_small_field, csrc/fz_compress.cu) against the oracle
-and against the list launches, byte for byte, around its edges: no full block, one block, items of
-16384 codes around 1, 2, 8, 15 and 16 of them (17 go to the other path), tails, fields longer than
-their dims, values past the 16-bit path; recorded in a graph; between larger fields of a batch."""
+"""Compression without a compaction launch (k_whole_field, csrc/fz_compress.cu) against the oracle,
+byte for byte, around its edges: no full block, one block, items of 16384 codes around 1, 2, 8, 15
+and 16 of them (the cluster's limit), tails, fields longer than their dims, values past the 16-bit
+path; up to and past one resident wave of items, against the list launches too; recorded in a graph;
+between larger fields of a batch."""
 import numpy as np
 import pytest
 import torch
@@ -71,3 +72,21 @@ def test_small_between_large(fz, oracle, ws):
     for _ in range(2):
         graph.replay()
         check()
+
+
+@pytest.mark.parametrize("dims", [(17 * 16384, 1, 1), (152 * 16384 + 5, 1, 1), (608 * 16384, 1, 1), (608 * 16384 + 1, 1, 1),
+                                  (2048, 456 * 8, 1), (2047, 456 * 8, 1), (2048, 456 * 8 + 1, 1), (128, 128, 456), (129, 127, 457),
+                                  (128, 129, 456)], ids=lambda d: "x".join(map(str, d)))
+def test_one_wave(fz, oracle, dims):
+    n = dims[0] * dims[1] * dims[2]
+    w = fz.Workspace(n)
+    for data in (field(n, 1, 50.0), np.abs(field(n, 2)), field(n, 3, 1e5)):
+        dev = torch.from_numpy(data).cuda()
+        listed = torch.zeros(fz.max_compressed_bytes(n, dims), dtype=torch.uint8, device="cuda")
+        for eb, rel, mode in ((1e-3, True, 1), (1e-2, False, 1), (1e-5, True, 0)):
+            want = oracle.compress(data, dims, eb, rel=rel, mode=mode)
+            got = fz.compress(dev, dims, eb, rel=rel, mode=mode, ws=w)
+            assert np.array_equal(got.cpu().numpy(), want), (eb, rel, mode)
+            fz.compress_batch(w, fz.fields_array([{"src": dev.data_ptr(), "dst": listed.data_ptr(), "n": n, "dims": dims,
+                                                   "eb": eb, "dst_capacity": listed.numel()}]), rel=rel, mode=mode)
+            assert np.array_equal(listed[:want.size].cpu().numpy(), want), (eb, rel, mode)
