@@ -432,7 +432,7 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     J.s2off   = group_sum_l2(ws->max_tiles);
     J.rel    = eb_mode == FZ_EB_REL;
     field_items(L.n, L.nb, a.ntiles, J.rel != 0, J.nr, J.ne, J.nc);
-    const bool small = J.ne <= kSmallItems, whole = small || (!ra && whole_field_fits((int)L.ndim, J.ne));
+    const bool small = J.ne <= kSmallItems, whole = small || (!ra && whole_field_fits((int)L.ndim, J.ne, out_bytes != nullptr));
     if (small || (ra && ra->have && J.rel)) J.nr = 0;  // the launch itself, or the previous call's encode launch, takes the range
     // range ahead: only when a compaction launch follows the encode launch (it moves the
     // accumulated range into place once every encode CTA has finished)

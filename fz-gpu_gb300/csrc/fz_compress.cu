@@ -1609,7 +1609,8 @@ __global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas<ND>)
 // -> 6.8 us, 362x362 (unaligned rows) 38.9 -> 33.8 / 14.2 -> 10.3, 512x512 37.0 -> 32.4 / 13.2 -> 9.0,
 // 64x64x64 35.9 -> 32.8 / 12.7 -> 9.5; in the float path (1e-5) 512x512 41.2 -> 34.3 / 17.3 -> 11.0.
 //
-// kScan true, after the range launch, at most one resident wave of items: items are handed out by
+// kScan true, after the range launch, at most one resident wave of items (half a wave when the caller
+// does not wait, whole_field_fits): items are handed out by
 // tickets, each CTA publishes its chunk count and sums the counts of all items before its own (their
 // CTAs have started, and wait for none after them).  Past one wave this loses: CTAs that wait hold
 // the memory the next items need, and all wait for the slowest (a persistent form of it took 43.7 us
@@ -1919,9 +1920,10 @@ static uint32_t whole_wave()
     return w;
 }
 
-bool whole_field_fits(int nd, uint32_t ne)
+bool whole_field_fits(int nd, uint32_t ne, bool waits)
 {
-    return ne <= (nd == 1 ? whole_wave<1, true>() : nd == 2 ? whole_wave<2, true>() : whole_wave<3, true>());
+    const uint32_t wave = nd == 1 ? whole_wave<1, true>() : nd == 2 ? whole_wave<2, true>() : whole_wave<3, true>();
+    return ne <= (waits ? wave : wave / 2);
 }
 
 template <int ND>

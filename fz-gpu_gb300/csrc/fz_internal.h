@@ -151,10 +151,16 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 
 // Single fields of at most this many encode items (16384 codes each) are compressed by one launch of
 // one cluster: the largest cluster there is, and at 16 items the launch still takes less time than
-// the three (figures at k_whole_field).  whole_field_fits: `ne` items are one resident wave of the
-// launch that follows a range launch.
+// the three (figures at k_whole_field).  whole_field_fits: whether the launch that follows a range
+// launch is to compress `ne` items whole.  Its CTAs hold their SMs until the counts before theirs are
+// in, so the limit is one resident wave where the caller waits for the size, and half of it, two
+// fields at once, where calls may follow each other on several streams.  GB300, 1 / 2 / 4 / 8 streams,
+// us a field, two launches -> one: 2000x1500 (184 items, waves of 456) 19.6 / 11.6 / 9.2 / 9.4 -> 15.3
+// / 9.1 / 8.5 / 7.4, but 2000x2200 (269) 21.0 / 12.1 / 9.4 / 9.4 -> 17.4 / 13.3 / 10.5 / 11.4; with a
+// size readback, 1 / 2 / 4 / 8 threads: 3600x1800 (396) 37.2 / 20.7 / 13.0 / 12.4 -> 34.9 / 18.9 / 13.2
+// / 14.0.
 constexpr uint32_t kSmallItems = 16;
-bool        whole_field_fits(int nd, uint32_t ne);
+bool        whole_field_fits(int nd, uint32_t ne, bool waits);
 cudaError_t launch_whole_field(int nd, const FieldJob& J, cudaStream_t s);
 
 // Items of each kind for a field of n elements (ntiles scan tiles of shuffle blocks, nb full
