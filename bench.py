@@ -944,6 +944,7 @@ def run_kernels(args, local_rank):
             assert torch.equal(na[: nb.value], out[fz.MODE_SIDECAR][: nb.value])
     torch.cuda.synchronize()
     print(json.dumps({"workload": WORKLOAD, "steps": args.steps,
+                      "note": "a field of at most one wave of CTAs: k_whole_field for encode and compaction",
                       "per_step": ["k_range_fields", "k_encode_fields", "k_compact_fields", "k_decompress (sidecar)",
                                    "k_range_fields", "k_encode_fields", "k_compact_fields", "k_offsets",
                                    "k_decompress (COMPAT)"] + (["k_range", "k_compress"] if noalloc else [])}),

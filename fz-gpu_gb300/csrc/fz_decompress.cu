@@ -402,9 +402,10 @@ __device__ __forceinline__ Pair delta2(uint32_t x)
 
 // Stores min(live, 4) reconstructed values at out (none for live <= 0).  kAl: all 4, 16-byte
 // aligned, as streaming stores: the field is written once and would push the stream out of the
-// L2 (GB300: 39200x388 18.7 -> 17.6 us, 1100x200x100 44.3 -> 39.5, 500x500x100 31.2 -> 30.4).  (Rows that start anywhere: gathering the aligned groups of 4 from neighbouring threads
-// by shuffle took more instructions than its wider stores saved, 501x500x100 on GB300 46.6 ->
-// 49.1 us.)
+// L2 (GB300: 39200x388 18.7 -> 17.6 us, 1100x200x100 44.3 -> 39.5, 500x500x100 31.2 -> 30.4).
+// (Rows that start anywhere: gathering the aligned groups of 4 from neighbouring threads by
+// shuffle took more instructions than its wider stores saved, 501x500x100 on GB300 46.6 -> 49.1
+// us.)
 template <bool kAl>
 __device__ __forceinline__ void store_row(float* out, int32_t live, Pair a, Pair b, float ebx2)
 {
@@ -453,8 +454,8 @@ __device__ __forceinline__ void sums_x(uint32_t x01, uint32_t x23, uint32_t q, P
 //
 // Bound by instruction issue (70%), then by the tail of a last wave.  GB300, event-timed, with
 // the signs undone in the bit planes, planes 7..14 left out where a warp has none, and the sums
-// in float pairs, against a sign per code and integer sums: 39200x388 20.7 -> 18.5 us,
-// 8192x8192 69.7 -> 57.5, 3601x1801 16.9 -> 14.6; 3600x1800 12.6 as with the separate kernel for
+// in float pairs, against a sign per code and integer sums: 39200x388 20.7 -> 18.5 us (17.6 with
+// the streaming stores), 8192x8192 69.7 -> 57.5, 3601x1801 16.9 -> 14.6; 3600x1800 12.6 as with the separate kernel for
 // x % 16 == 0 (12.3-13.0) that it replaces.  256 threads, 4 CTAs an SM (64 registers): 5 CTAs of
 // 48 registers spill (3600x1800 13.5 us, 39200x388 18.8, 8192x8192 56.1); 128 threads with
 // 448-column windows lose as much to the groups shared between windows (14.1, 19.0, 59.5).
