@@ -98,6 +98,7 @@ SIGNATURES = {
     "fz_workspace_bytes": (_I, [_U64, _PU64]),
     "fz_workspace_status": (_I, [_P, _P]),
     "fz_selftest_wait_timeout": (_I, [_P, _P]),
+    "fz_selftest_whole_timeout": (_I, [_P, _P, _U64, Dims, _D, _I, _I, _P, _U64, _U32, _PU64, _P]),
     "fz_workspace_enable_timing": (_I, [_P, _U32]),
     "fz_workspace_kernel_time": (_I, [_P, _I, C.POINTER(C.c_uint32), C.POINTER(C.c_double)]),
     "fz_compress": (_I, [_P, _P, _U64, Dims, _D, _I, _I, _P, _U64, _PU64, _P]),
@@ -230,6 +231,13 @@ class Workspace:
     def selftest_wait_timeout(self, stream=None):
         """Status of a look-back that waits on a tile nothing publishes (FZ_TIMEOUT)."""
         return lib().fz_selftest_wait_timeout(self.handle, _stream_handle(stream))
+
+    def selftest_whole_timeout(self, x, dims, eb, item, out, rel=True, mode=MODE_SIDECAR, readback=True, stream=None):
+        """Status of a compression in which item `item`'s wait counts as run out (FZ_TIMEOUT with readback)."""
+        n = C.c_uint64()
+        return lib().fz_selftest_whole_timeout(self.handle, x.data_ptr(), x.numel(), _dims(dims), float(eb),
+                                               EB_REL if rel else EB_ABS, mode, out.data_ptr(), out.numel(), item,
+                                               C.byref(n) if readback else None, _stream_handle(stream))
 
     # timing kinds of fz_workspace_kernel_time, by the kernels they time:
     # k_encode_fields<ND> and k_decompress{1,2,3}d are templated / specialised per

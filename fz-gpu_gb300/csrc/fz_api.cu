@@ -401,7 +401,8 @@ static fz_status read_size(fz_workspace* ws, const Layout& L, const uint32_t* mi
 // written by the last kernel; the request loop reads both with one copy).
 fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_dims dims, double eb,
                             fz_eb_mode eb_mode, fz_mode mode, void* d_out, uint64_t out_capacity,
-                            uint64_t* out_bytes, fz_stream_t stream, uint32_t* mirror, RangeAhead* ra)
+                            uint64_t* out_bytes, fz_stream_t stream, uint32_t* mirror, RangeAhead* ra,
+                            const uint32_t* give_up)
 {
     if (ra) ra->done = false;
     if (!ws) return FZ_INVALID_ARG;
@@ -428,11 +429,16 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     J.slots  = reinterpret_cast<uint4*>(ws->codes);
     J.counts = ws->boff;
     J.supers = ws->supers;
+    J.whole  = reinterpret_cast<uint64_t*>(ws->tickets + 8);
     J.sstride = group_sum_words(ws->max_tiles);
     J.s2off   = group_sum_l2(ws->max_tiles);
     J.rel    = eb_mode == FZ_EB_REL;
     field_items(L.n, L.nb, a.ntiles, J.rel != 0, J.nr, J.ne, J.nc);
     const bool small = J.ne <= kSmallItems, whole = small || (!ra && whole_field_fits((int)L.ndim, J.ne, out_bytes != nullptr));
+    if (give_up) {
+        if (small || !whole || *give_up >= J.ne) return FZ_INVALID_ARG;
+        J.give_up = *give_up;
+    }
     if (small || (ra && ra->have && J.rel)) J.nr = 0;  // the launch itself, or the previous call's encode launch, takes the range
     // range ahead: only when a compaction launch follows the encode launch (it moves the
     // accumulated range into place once every encode CTA has finished)
@@ -597,6 +603,14 @@ fz_status fz_selftest_wait_timeout(fz_workspace* ws, fz_stream_t stream)
     cudaError_t r = launch_wait_selftest(ws->state, ws->epoch, ws->status, s);
     if (r != cudaSuccess) return map_err(r);
     return fz_workspace_status(ws, stream);
+}
+
+fz_status fz_selftest_whole_timeout(fz_workspace* ws, const float* d_in, uint64_t n, fz_dims dims, double eb,
+                                    fz_eb_mode eb_mode, fz_mode mode, void* d_out, uint64_t out_capacity, uint32_t item,
+                                    uint64_t* out_bytes, fz_stream_t stream)
+{
+    return fz::compress_impl(ws, d_in, n, dims, eb, eb_mode, mode, d_out, out_capacity, out_bytes, stream, nullptr,
+                             nullptr, &item);
 }
 
 // ------------------------------------------------------------------ stages --

@@ -1597,8 +1597,19 @@ __global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas<ND>)
     }
 }
 
+// J.whole of k_whole_field<ND, true>, one add an item once its wait is over: items counted [0, 16),
+// waits that gave up [16, 32), the last item's chunk total [32, 61) and whether a code overflowed
+// (bit 63).  A wait that gave up leaves out its item's chunks, whatever the last item's own wait
+// did, so the thread that counts last, which knows of every wait, writes the header (no fence:
+// all it needs is in the word).
+__device__ __forceinline__ uint64_t wait_word(bool ok, bool last, uint32_t total, uint32_t ovf)
+{
+    return (ok ? 1u : 0x10001u) | (last ? ((uint64_t)total << 32) | ((uint64_t)(ovf != 0) << 63) : 0u);
+}
+
 // A whole field in one launch of one CTA per encode item; the chunks go from the images straight to
-// Section B, with no slots, group sums or compaction launch; the last item's CTA writes the header.
+// Section B, with no slots, group sums or compaction launch; the last item's CTA (kScan: the one whose
+// wait ends last) writes the header.
 //
 // kScan false, at most kSmallItems items: the CTAs are one cluster.  Each takes the max/min of its
 // item's elements, they exchange them through distributed shared memory, each encodes its item, and
@@ -1612,7 +1623,7 @@ __global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas<ND>)
 // kScan true, after the range launch, at most one resident wave of items (half a wave when the caller
 // does not wait, whole_field_fits): items are handed out by
 // tickets, each CTA publishes its chunk count and sums the counts of all items before its own (their
-// CTAs have started, and wait for none after them).  Past one wave this loses: CTAs that wait hold
+// CTAs have started, and wait for none after them; a wait gives up after kSpinLimit / 16 rounds).  Past one wave this loses: CTAs that wait hold
 // the memory the next items need, and all wait for the slowest (a persistent form of it took 43.7 us
 // for the 928 items of 39200x388, the encode and compaction launches 23.5 and 8).  Two launches ->
 // this one, same measures: 1000x1000 38.8 -> 35.3 / 13.6 -> 11.5, 3600x1800 47.4 -> 42.9 / 21.4 ->
@@ -1620,6 +1631,10 @@ __global__ void __launch_bounds__(kCompressWarps * 32, kEncodeCtas<ND>)
 // 42.7 -> 40.9 / 15.9 -> 16.0 (184 items: 32 of the 152 SMs have two).  A polling thread per count
 // instead of one polling warp: 4000000 in a graph 18.5.  A cooperative launch with the range inside,
 // behind a grid barrier, was no faster than the range launch and cannot overlap its neighbours.
+//
+// The count of ended waits (wait_word), an atomic whose way the chunk stores cover, costs 0 to 0.5 us:
+// in a graph 3600x1800 21.3 and 21.3 us without and with it, 1000x1000 11.6 and 11.7, 2000x1500 15.5 and 15.9.
+// The header written before the count, with a release: 1.5 to 2 us where its mirror is host memory.
 template <int ND, bool kScan>
 __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_whole_field(const __grid_constant__ FieldJob J)
 {
@@ -1701,13 +1716,16 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_whole_field(const __
             if (kScan) publish(a.state, item, s_epoch, kFlagAgg, ovf ? 1u : 0u, tot);
         }
     }
-    uint32_t        excl, prior = 0, pt = 0;
+    uint32_t        excl, pt = 0;
     const uint32_t* peer = nullptr;
     bool            ok   = true;
+    uint64_t        counted = 0;
+    FieldFinal      fin{};
     if constexpr (kScan) {
         // the counts of all items before this one: their CTAs took their tickets earlier and wait for
         // no later one.  One warp polls, four loads a lane in flight.
         if (wid == 0) {
+            if (lane == 0) fin = final_loads(J);  // (final since the range launch; for the thread that counts last)
             uint32_t v, o, spins = 0;
             bool     all;
             do {
@@ -1729,11 +1747,17 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_whole_field(const __
                 if (!all) __nanosleep(40);  // (polls of many CTAs hold up the counts' way through the L2)
             } while (!all && ++spins <= kSpinLimit / 16);  // (a round polls up to 20 words a lane)
             v = __reduce_add_sync(kFull, v), o = __reduce_or_sync(kFull, o);
-            if (lane == 0) s_excl = v, s_prior = o, s_ok = all;
+            all = all && item != J.give_up;
+            if (lane == 0) s_excl = v, s_ok = all;
+            if (lane == 0) s_prior = o;
         }
         __syncthreads();
-        excl = s_excl, prior = s_prior, ok = s_ok != 0;
-        if (!ok && tid == 0) atomicOr(a.status, kStatusTimeout);
+        excl = s_excl, ok = s_ok != 0;
+        if (tid == 0) {
+            if (!ok) atomicOr(a.status, kStatusTimeout);
+            const uint64_t add = wait_word(ok, item == items - 1, excl + s_tot[0], s_prior | s_tot[1]);
+            counted            = atomicAdd(reinterpret_cast<unsigned long long*>(J.whole), add) + add;
+        }
     } else {
         cluster.sync();
         peer = lane < items ? cluster.map_shared_rank(s_tot, lane) : nullptr;
@@ -1754,28 +1778,28 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_whole_field(const __
             pre += __popc(c.bm[u]);
         }
     }
-    if (item == items - 1 && wid == 0) {
-        if constexpr (kScan) {
-            if (lane == 0) {
-                FieldFinal fin = final_loads(J);
-                if (prior | s_tot[1]) fin.flags |= kCtlOverflow;
-                if (!ok) fin.flags |= kStatusNonfinite, fin.status |= kStatusTimeout;  // marks the stream failed
-                finish_field(J, excl + s_tot[0], fin);
-            }
-        } else {
-            const uint32_t total = __reduce_add_sync(kFull, pt), ovf = __reduce_or_sync(kFull, peer ? peer[1] : 0u);
-            if (lane == 0) {
-                const uint32_t st = s_bad ? atomicOr(a.status, kStatusNonfinite) | kStatusNonfinite : a.mirror ? __ldcg(a.status) : 0u;
-                write_header(a, s_eb, (ovf ? 1u : 0u) | (s_bad ? 2u : 0u), total, reinterpret_cast<uint4*>(a.mirror));
-                if (a.mirror) a.mirror[16] = st;
-                if (a.boff) {
-                    a.boff[a.nb] = total;  // the total closes the offset table; zero its 16-byte pad
-                    for (uint32_t k = a.nb + 1; k < (uint32_t)(pad16(4ull * (a.nb + 1)) / 4); ++k) a.boff[k] = 0;
-                }
+    if (!kScan && item == items - 1 && wid == 0) {
+        const uint32_t total = __reduce_add_sync(kFull, pt), ovf = __reduce_or_sync(kFull, peer ? peer[1] : 0u);
+        if (lane == 0) {
+            const uint32_t st = s_bad ? atomicOr(a.status, kStatusNonfinite) | kStatusNonfinite : a.mirror ? __ldcg(a.status) : 0u;
+            write_header(a, s_eb, (ovf ? 1u : 0u) | (s_bad ? 2u : 0u), total, reinterpret_cast<uint4*>(a.mirror));
+            if (a.mirror) a.mirror[16] = st;
+            if (a.boff) {
+                a.boff[a.nb] = total;  // the total closes the offset table; zero its 16-byte pad
+                for (uint32_t k = a.nb + 1; k < (uint32_t)(pad16(4ull * (a.nb + 1)) / 4); ++k) a.boff[k] = 0;
             }
         }
     }
-    if (!kScan) cluster.sync();  // no CTA leaves while another reads its counts
+    if constexpr (kScan) {
+        if (tid == 0 && (counted & 0xFFFFu) == items) {
+            *J.whole = 0;
+            if (counted >> 63) fin.flags |= kCtlOverflow;
+            if (counted & 0xFFFF0000u) fin.flags |= kStatusNonfinite, fin.status |= kStatusTimeout;  // marks the stream failed
+            finish_field(J, (uint32_t)(counted >> 32) & 0x1FFFFFFFu, fin);
+        }
+    } else {
+        cluster.sync();  // no CTA leaves while another reads its counts
+    }
 }
 
 template <bool kList>
@@ -1923,7 +1947,7 @@ static uint32_t whole_wave()
 bool whole_field_fits(int nd, uint32_t ne, bool waits)
 {
     const uint32_t wave = nd == 1 ? whole_wave<1, true>() : nd == 2 ? whole_wave<2, true>() : whole_wave<3, true>();
-    return ne <= (waits ? wave : wave / 2);
+    return ne <= std::min(waits ? wave : wave / 2, 0xFFFFu);  // (wait_word counts in 16 bits)
 }
 
 template <int ND>

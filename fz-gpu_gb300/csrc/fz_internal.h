@@ -92,6 +92,10 @@ struct FieldJob {
     // encode items; ahead_nr == 0: none
     const float* ahead_in;
     uint32_t     ahead_n, ahead_nr;
+    // k_whole_field after a range launch: its count of ended waits (zero on entry, left zero), and the
+    // item whose wait counts as run out (fz_selftest_whole_timeout), ~0: none
+    uint64_t* whole   = nullptr;
+    uint32_t  give_up = ~0u;
 };
 
 // Items [start, start + count) of a list launch belong to field `field` (its items 0 ..

@@ -13,7 +13,7 @@ struct fz_workspace {
     void*     d_base;
     size_t    d_bytes;
     uint64_t* state;
-    uint32_t* tickets;  // [0] look-back compress, [1] offsets, [2] scan-encode, [3] unused
+    uint32_t* tickets;  // [0] k_whole_field, [1] offsets, [2] scan-encode, [8..9] FieldJob::whole
     uint32_t* status;
     uint32_t* total;
     uint32_t* epoch;    // device epoch of the scan state
@@ -44,8 +44,10 @@ struct RangeAhead {
     bool            done = false;    // out: the range of `next` was accumulated
 };
 // fz_compress with an optional device mirror (128 bytes, 16-byte aligned) that receives
-// the 64-byte header and, at word 16, the status word once the stream is complete.
+// the 64-byte header and, at word 16, the status word once the stream is complete.  give_up
+// (self-test): FieldJob::give_up; FZ_INVALID_ARG where the call has no such wait.
 fz_status compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_dims dims, double eb,
                         fz_eb_mode eb_mode, fz_mode mode, void* d_out, uint64_t out_capacity,
-                        uint64_t* out_bytes, fz_stream_t stream, uint32_t* mirror, RangeAhead* ra = nullptr);
+                        uint64_t* out_bytes, fz_stream_t stream, uint32_t* mirror, RangeAhead* ra = nullptr,
+                        const uint32_t* give_up = nullptr);
 }  // namespace fz

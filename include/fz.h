@@ -167,6 +167,14 @@ fz_status fz_workspace_kernel_time(fz_workspace* ws, int kind, uint32_t* launche
    call returns FZ_TIMEOUT; any other result means the wait bound is broken.  No
    reference counterpart (the reference's only device-wide step is a CUB scan). */
 fz_status fz_selftest_wait_timeout(fz_workspace* ws, fz_stream_t stream);
+/* Diagnostic: fz_compress of a field that takes encode and compaction in one launch after the
+   range launch (FZ_INVALID_ARG for others), in which encode item `item` (16384 codes) behaves
+   as if its wait for the chunk counts before its own had run out: its chunks are left out.
+   The header must carry FZ_FLAG_FAILED, and a call with out_bytes returns FZ_TIMEOUT. */
+fz_status fz_selftest_whole_timeout(fz_workspace* ws, const float* d_in, uint64_t n, fz_dims dims,
+                                    double eb, fz_eb_mode eb_mode, fz_mode mode, void* d_out,
+                                    uint64_t out_capacity, uint32_t item, uint64_t* out_bytes,
+                                    fz_stream_t stream);
 
 /* ------------------------------------------------ full pipeline, device -- */
 /* Compress d_in[0..n) (dims describe the first x*y*z elements; n may exceed it as

@@ -1,0 +1,56 @@
+"""Encode and compaction in one launch after the range launch (k_whole_field<ND, true>): a wait that
+gave up marks the stream whichever item it was."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ITEM = 16384
+
+
+def field(n, seed):
+    rng = np.random.default_rng(seed)
+    return (np.cumsum(rng.standard_normal(n)) / np.sqrt(n)).astype(np.float32)
+
+
+def wave(nd):
+    """Items of one resident wave: 4 CTAs an SM in 1D, 3 otherwise."""
+    return torch.cuda.get_device_properties(0).multi_processor_count * (4 if nd == 1 else 3)
+
+
+def dims_of(nd, items):
+    return [(items * ITEM, 1, 1), (256, 64 * items, 1), (64, 64, 4 * items)][nd - 1]
+
+
+@pytest.mark.parametrize("nd", [1, 2, 3])
+@pytest.mark.parametrize("where", ["first", "second", "middle", "last"])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_given_up_wait_marks_the_stream(fz, oracle, nd, where, mode):
+    items = 40
+    dims, item = dims_of(nd, items), {"first": 0, "second": 1, "middle": items // 2, "last": items - 1}[where]
+    data = field(items * ITEM, nd)
+    x, ws = torch.from_numpy(data).cuda(), fz.Workspace(items * ITEM)
+    out = torch.zeros(fz.max_compressed_bytes(x.numel(), dims, mode), dtype=torch.uint8, device="cuda")
+    want = oracle.compress(data, dims, 1e-3, rel=True, mode=mode)
+    for readback in (True, False):
+        assert ws.selftest_whole_timeout(x, dims, 1e-3, item, out, mode=mode, readback=readback) == (
+            fz.TIMEOUT if readback else fz.SUCCESS)
+        torch.cuda.synchronize()
+        assert fz.parse_header(out[:64].cpu().numpy()).flags & 2
+        with pytest.raises(fz.FzError):
+            fz.decompress(out, ws=ws)
+        assert ws.status() == (fz.SUCCESS if readback else fz.TIMEOUT)
+        # the next call on the workspace is as any other
+        got = fz.compress(x, dims, 1e-3, mode=mode, ws=ws, out=out)
+        assert np.array_equal(got.cpu().numpy(), want)
+        assert fz.parse_header(got[:64].cpu().numpy()).flags & 2 == 0
+
+
+def test_no_wait_to_give_up(fz):
+    """Fields of one cluster, or past one wave, have no such wait; nor does an item past the last."""
+    for items, item in ((16, 3), (40, 40), (wave(2) + 1, 3)):
+        dims = dims_of(2, items)
+        x, ws = torch.ones(items * ITEM, device="cuda"), fz.Workspace(items * ITEM)
+        out = torch.zeros(fz.max_compressed_bytes(x.numel(), dims), dtype=torch.uint8, device="cuda")
+        assert ws.selftest_whole_timeout(x, dims, 1e-3, item, out) == fz.INVALID_ARG
