@@ -117,6 +117,15 @@ fz_status take_status(fz_workspace* ws, uint32_t st, cudaStream_t s)
     return FZ_SUCCESS;
 }
 
+// The status word (syncs).
+cudaError_t fetch_status(fz_workspace* ws, cudaStream_t s, uint32_t& st)
+{
+    cudaError_t e = cudaMemcpyAsync(ws->h_pinned + 64, ws->status, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    std::memcpy(&st, ws->h_pinned + 64, 4);
+    return e;
+}
+
 fz_status validate_header(const fz_header* h, uint64_t stream_bytes, Layout* out)
 {
     if (h->magic != FZ_MAGIC || h->version != FZ_FORMAT_VERSION) return FZ_CORRUPT_STREAM;
@@ -328,12 +337,9 @@ fz_status fz_workspace_status(fz_workspace* ws, fz_stream_t stream)
 {
     if (!ws) return FZ_INVALID_ARG;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    cudaError_t  e = cudaMemcpyAsync(ws->h_pinned + 64, ws->status, 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
-    uint32_t st;
-    std::memcpy(&st, ws->h_pinned + 64, 4);
-    return take_status(ws, st, s);
+    uint32_t     st;
+    cudaError_t  e = fetch_status(ws, s, st);
+    return e == cudaSuccess ? take_status(ws, st, s) : map_err(e, FZ_FAIL_GPU_MEMCPY);
 }
 
 fz_status fz_compress(fz_workspace* ws, const float* d_in, uint64_t n, fz_dims dims, double eb,
@@ -663,12 +669,13 @@ fz_status fz_scan_encode(fz_workspace* ws, const uint8_t* d_shuffled, const uint
     if (e != cudaSuccess) return map_err(e);
     if (nnz) {
         e = cudaMemcpyAsync(ws->h_pinned, ws->total, 4, cudaMemcpyDeviceToHost, s);
+        uint32_t bits;
+        if (e == cudaSuccess) e = fetch_status(ws, s, bits);  // (syncs)
         if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
-        st = fz_workspace_status(ws, stream);  // (syncs)
         uint32_t t;
         std::memcpy(&t, ws->h_pinned, 4);
         *nnz = t;
-        return st;
+        return take_status(ws, bits, s);
     }
     return FZ_SUCCESS;
 }

@@ -1,0 +1,68 @@
+"""The library's host code (csrc/fz_api.cu) on a CUDA runtime that fails where it is told to
+(fake_cuda.cu): no GPU, no kernel."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA_ERROR = 719  # cudaErrorLaunchFailure
+
+
+@pytest.fixture(scope="module")
+def api(fz, tmp_path_factory):
+    import __graft_entry__ as g
+    b = g._load_build_module()
+    os.makedirs(b.BUILD, exist_ok=True)
+    obj = b.compile_one("fz_api.cu")
+    d = tmp_path_factory.mktemp("fake")
+    src, so = os.path.join(HERE, "fake_cuda.cpp"), str(d / "libfzhost.so")
+    runtime, launchers = str(d / "runtime.o"), str(d / "launchers.o")
+    subprocess.check_call(["g++", "-std=c++17", "-fPIC", "-I" + os.path.join(b.cuda_home(), "include"), "-c", src, "-o", runtime])
+    subprocess.check_call([b.nvcc()] + b.ARCH + b.NVCC_FLAGS + ["-x", "cu", "-c", src, "-o", launchers])
+    subprocess.check_call(["g++", "-shared", "-Wl,-Bsymbolic", "-o", so, obj, runtime, launchers])
+    L = C.CDLL(so)
+    for name, (res, args) in fz.SIGNATURES.items():
+        if hasattr(L, name):
+            f = getattr(L, name)
+            f.restype, f.argtypes = res, args
+    L.fake_calls.restype = C.c_char_p
+    L.fake_fail.argtypes = [C.c_char_p, C.c_int, C.c_int]
+    return L
+
+
+@pytest.fixture
+def ws(api, fz):
+    h = C.c_void_p()
+    assert api.fz_workspace_create(1 << 20, C.byref(h)) == fz.SUCCESS
+    api.fake_reset()
+    yield h
+    api.fake_reset()
+    api.fz_workspace_destroy(h)
+
+
+def aligned(n, dtype):
+    raw = np.zeros(n * np.dtype(dtype).itemsize + 16, np.uint8)
+    off = -raw.ctypes.data % 16
+    return raw[off:off + n * np.dtype(dtype).itemsize].view(dtype)
+
+
+def calls(api):
+    return api.fake_calls().decode().split()
+
+
+@pytest.mark.parametrize("call,nth", [(b"cudaMemcpyAsync", 1), (b"cudaMemcpyAsync", 2), (b"cudaStreamSynchronize", 1)])
+def test_scan_encode_total_only_when_read(api, fz, ws, call, nth):
+    """The chunk total is stored only after the wait that brought it."""
+    n = 4096
+    shuffled, flags = aligned(2 * n, np.uint8), aligned(n // 8, np.uint32)
+    nnz = C.c_uint64(123456789)
+    api.fake_fail(call, nth, CUDA_ERROR)
+    st = api.fz_scan_encode(ws, shuffled.ctypes.data, flags.ctypes.data, n, None, None, C.byref(nnz), None)
+    assert st != fz.SUCCESS
+    assert nnz.value == 123456789
+    api.fake_reset()
+    assert api.fz_scan_encode(ws, shuffled.ctypes.data, flags.ctypes.data, n, None, None, C.byref(nnz), None) == fz.SUCCESS
+    assert nnz.value == 7
