@@ -117,13 +117,21 @@ fz_status take_status(fz_workspace* ws, uint32_t st, cudaStream_t s)
     return FZ_SUCCESS;
 }
 
-// The status word (syncs).
+// The status word.  Waits for the stream whether or not the word's copy starts: no copy enqueued
+// before is under way when the caller returns.
 cudaError_t fetch_status(fz_workspace* ws, cudaStream_t s, uint32_t& st)
 {
-    cudaError_t e = cudaMemcpyAsync(ws->h_pinned + 64, ws->status, 4, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const cudaError_t e = cudaMemcpyAsync(ws->h_pinned + 64, ws->status, 4, cudaMemcpyDeviceToHost, s);
+    const cudaError_t w = cudaStreamSynchronize(s);
     std::memcpy(&st, ws->h_pinned + 64, 4);
-    return e;
+    return e != cudaSuccess ? e : w;
+}
+
+// `st` once the copies of the caller's buffers that a failing call has enqueued are over.
+fz_status settled(cudaStream_t s, fz_status st)
+{
+    if (st != FZ_SUCCESS) (void)cudaStreamSynchronize(s);
+    return st;
 }
 
 fz_status validate_header(const fz_header* h, uint64_t stream_bytes, Layout* out)
@@ -568,7 +576,7 @@ fz_status fz_compress_host(fz_workspace* ws, const float* h_in, uint64_t n, fz_d
     if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
     uint64_t bytes = 0;
     st = fz_compress(ws, ws->d_field, n, dims, eb, eb_mode, mode, ws->d_stream, ws->stream_cap, &bytes, stream);
-    if (st != FZ_SUCCESS) return st;
+    if (st != FZ_SUCCESS) return settled(s, st);
     if (bytes > out_capacity) return FZ_OUT_OF_SPACE;
     e = cudaMemcpyAsync(h_out, ws->d_stream, bytes, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -593,9 +601,9 @@ fz_status fz_decompress_host(fz_workspace* ws, const void* h_stream, uint64_t st
     cudaError_t  e = cudaMemcpyAsync(ws->d_stream, h_stream, stream_bytes, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
     st = fz_decompress(ws, ws->d_stream, stream_bytes, &h, ws->d_field, ws->max_n, stream);
-    if (st != FZ_SUCCESS) return st;
+    if (st != FZ_SUCCESS) return settled(s, st);
     e = cudaMemcpyAsync(h_out, ws->d_field, 4 * h.n, cudaMemcpyDeviceToHost, s);
-    if (e != cudaSuccess) return map_err(e, FZ_FAIL_GPU_MEMCPY);
+    if (e != cudaSuccess) return settled(s, map_err(e, FZ_FAIL_GPU_MEMCPY));
     return fz_workspace_status(ws, stream);  // (syncs: one wait for the field and the status)
 }
 

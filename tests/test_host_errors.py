@@ -66,3 +66,25 @@ def test_scan_encode_total_only_when_read(api, fz, ws, call, nth):
     api.fake_reset()
     assert api.fz_scan_encode(ws, shuffled.ctypes.data, flags.ctypes.data, n, None, None, C.byref(nnz), None) == fz.SUCCESS
     assert nnz.value == 7
+
+
+@pytest.mark.parametrize("nth", [0, 1, 2, 3])
+def test_decompress_host_leaves_no_copy_under_way(api, fz, oracle, ws, nth):
+    """Whichever copy fails to start, none of the caller's buffers is in use once the call has returned."""
+    x = np.linspace(0, 1, 9000, dtype=np.float32)
+    stream = oracle.compress(x, (9000, 1, 1), 1e-3, rel=True, mode=1)
+    src, out = aligned(stream.size, np.uint8), np.zeros(x.size, np.float32)
+    src[:] = stream
+    if nth:
+        api.fake_fail(b"cudaMemcpyAsync", nth, CUDA_ERROR)
+    st = api.fz_decompress_host(ws, src.ctypes.data, src.size, out.ctypes.data, out.size, None)
+    assert (st == fz.SUCCESS) == (nth == 0)
+    assert api.fake_pending() == 0
+
+
+def test_compress_host_leaves_no_copy_under_way(api, fz, ws):
+    """A bound that the compression refuses after the field's copy has been enqueued."""
+    x, out = aligned(9000, np.float32), aligned(1 << 16, np.uint8)
+    st = api.fz_compress_host(ws, x.ctypes.data, x.size, fz.Dims(9000, 1, 1), -1.0, fz.EB_REL, 1, out.ctypes.data, out.size, None, None)
+    assert st == fz.INVALID_ARG
+    assert api.fake_pending() == 0
