@@ -448,7 +448,8 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     J.s2off   = group_sum_l2(ws->max_tiles);
     J.rel    = eb_mode == FZ_EB_REL;
     field_items(L.n, L.nb, a.ntiles, J.rel != 0, J.nr, J.ne, J.nc);
-    const bool small = J.ne <= kSmallItems, whole = small || (!ra && whole_field_fits((int)L.ndim, J.ne, out_bytes != nullptr));
+    const uint32_t clustered = small_items((int)L.ndim);
+    const bool small = J.ne <= clustered, whole = small || (!ra && whole_field_fits((int)L.ndim, J.ne, out_bytes != nullptr));
     if (give_up) {
         if (small || !whole || *give_up >= J.ne) return FZ_INVALID_ARG;
         J.give_up = *give_up;
@@ -464,7 +465,7 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
                                               f.dst_capacity, ws->status, Ln, an) == FZ_SUCCESS) {
             uint32_t nr, ne, nc;
             field_items(Ln.n, Ln.nb, an.ntiles, true, nr, ne, nc);
-            if (ne > kSmallItems) J.ahead_nr = nr, J.ahead_in = an.in, J.ahead_n = an.n;
+            if (ne > small_items((int)Ln.ndim)) J.ahead_nr = nr, J.ahead_in = an.in, J.ahead_n = an.n;
         }
     }
     cudaError_t e = cudaSuccess;

@@ -11,7 +11,7 @@
 //                     cub::DeviceScan, fz.cu:187-201) from per-group sums, the move of the
 //                     chunks to their final offsets, the offset table and the header.
 //   k_whole_field     the three in one launch for a single field: of one cluster, range
-//                     included, up to kSmallItems encode items; after a range launch, up to
+//                     included, up to small_items() encode items; after a range launch, up to
 //                     one resident wave of items.
 //   k_range, k_compress  the same forward path with a decoupled look-back over scan
 //                     tiles in a single persistent launch after a range pass; used where no
@@ -1611,7 +1611,7 @@ __device__ __forceinline__ uint64_t wait_word(bool ok, bool last, uint32_t total
 // Section B, with no slots, group sums or compaction launch; the last item's CTA (kScan: the one whose
 // wait ends last) writes the header.
 //
-// kScan false, at most kSmallItems items: the CTAs are one cluster.  Each takes the max/min of its
+// kScan false, at most small_items() items: the CTAs are one cluster.  Each takes the max/min of its
 // item's elements, they exchange them through distributed shared memory, each encodes its item, and
 // they exchange the chunk counts.  No word of the workspace but the status is used.  A field this
 // small is bound by latencies: three launches, each followed by the first loads of the next, the
@@ -1926,27 +1926,59 @@ cudaError_t launch_fields(FieldPhase phase, int nd, const FieldJob* jobs, const 
     }
 }
 
-// CTAs of one resident wave of k_whole_field<ND, kScan> on the current device (0: error), opted in to
-// its dynamic shared memory and to clusters past 8 CTAs.
-template <int ND, bool kScan>
+// `query` on the current device, kept per device once it is not 0 (an error).
+template <typename Q>
+static uint32_t per_device(std::atomic<uint32_t> (&known)[64], Q query)
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::atomic<uint32_t>* slot = dev < 64 ? &known[dev] : nullptr;
+    uint32_t               v    = slot ? slot->load(std::memory_order_acquire) : 0;
+    if (v) return v;
+    v = query();
+    if (slot) slot->store(v, std::memory_order_release);
+    return v;
+}
+
+// CTAs of one resident wave of k_whole_field<ND, true> on the current device (0: error), opted in to
+// its dynamic shared memory.
+template <int ND>
 static uint32_t whole_wave()
 {
     static std::atomic<uint32_t> waves[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    std::atomic<uint32_t>* slot = dev < 64 ? &waves[dev] : nullptr;
-    uint32_t               w    = slot ? slot->load(std::memory_order_acquire) : 0;
-    if (w) return w;
-    if (!kScan && cudaFuncSetAttribute(k_whole_field<ND, kScan>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        return 0;
-    w = resident_ctas(k_whole_field<ND, kScan>, kCompressWarps * 32, encode_smem<ND>());
-    if (slot) slot->store(w, std::memory_order_release);
-    return w;
+    return per_device(waves, [] { return resident_ctas(k_whole_field<ND, true>, kCompressWarps * 32, encode_smem<ND>()); });
 }
+
+// The largest cluster of k_whole_field<ND, false>, at most kSmallItems CTAs, that the current device
+// can place (0: error), opted in to its dynamic shared memory and to clusters past 8 CTAs.
+template <int ND>
+static uint32_t largest_cluster()
+{
+    static std::atomic<uint32_t> sizes[64];
+    return per_device(sizes, [] {
+        auto* const k = k_whole_field<ND, false>;
+        if (!resident_ctas(k, kCompressWarps * 32, encode_smem<ND>())) return 0u;
+        const bool wide = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        for (uint32_t c = wide ? kSmallItems : std::min(8u, kSmallItems); c > 1; --c) {
+            cudaLaunchAttribute at{};
+            at.id             = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim = {c, 1, 1};
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(c), cfg.blockDim = dim3(kCompressWarps * 32), cfg.dynamicSmemBytes = encode_smem<ND>();
+            cfg.attrs = &at, cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0) return c;
+            (void)cudaGetLastError();  // a size that is refused leaves no error behind
+        }
+        return 1u;
+    });
+}
+
+uint32_t small_items(int nd) { return nd == 1 ? largest_cluster<1>() : nd == 2 ? largest_cluster<2>() : largest_cluster<3>(); }
 
 bool whole_field_fits(int nd, uint32_t ne, bool waits)
 {
-    const uint32_t wave = nd == 1 ? whole_wave<1, true>() : nd == 2 ? whole_wave<2, true>() : whole_wave<3, true>();
+    const uint32_t wave = nd == 1 ? whole_wave<1>() : nd == 2 ? whole_wave<2>() : whole_wave<3>();
     return ne <= std::min(waits ? wave : wave / 2, 0xFFFFu);  // (wait_word counts in 16 bits)
 }
 
@@ -1954,8 +1986,7 @@ template <int ND>
 static cudaError_t launch_whole(const FieldJob& J, cudaStream_t s)
 {
     const dim3 grid(J.ne), block(kCompressWarps * 32);
-    if (J.ne > kSmallItems) return launch_pdl(k_whole_field<ND, true>, grid, block, encode_smem<ND>(), s, J);
-    if (!whole_wave<ND, false>()) return cudaErrorInvalidDevice;
+    if (J.ne > largest_cluster<ND>()) return launch_pdl(k_whole_field<ND, true>, grid, block, encode_smem<ND>(), s, J);
     return launch_pdl_cluster(k_whole_field<ND, false>, grid, block, encode_smem<ND>(), s, J.ne, J);
 }
 

@@ -163,7 +163,10 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 // / 9.1 / 8.5 / 7.4, but 2000x2200 (269) 21.0 / 12.1 / 9.4 / 9.4 -> 17.4 / 13.3 / 10.5 / 11.4; with a
 // size readback, 1 / 2 / 4 / 8 threads: 3600x1800 (396) 37.2 / 20.7 / 13.0 / 12.4 -> 34.9 / 18.9 / 13.2
 // / 14.0.
+// small_items: kSmallItems, or the largest cluster that the current device can place, where that is
+// smaller (16 is past the portable size of 8; the CTAs of one share a GPC).
 constexpr uint32_t kSmallItems = 16;
+uint32_t    small_items(int nd);
 bool        whole_field_fits(int nd, uint32_t ne, bool waits);
 cudaError_t launch_whole_field(int nd, const FieldJob& J, cudaStream_t s);
 

@@ -86,6 +86,8 @@ void field_items(uint32_t n, uint32_t nb, uint32_t ntiles, bool rel, uint32_t& n
 {
     nr = rel ? (uint32_t)cdiv(n, 1024) : 0u, ne = (uint32_t)cdiv(ntiles, 8), nc = (uint32_t)cdiv(nb, 32);
 }
+uint32_t    fake_cluster = 16;
+uint32_t    small_items(int) { return fake_cluster; }
 bool        whole_field_fits(int, uint32_t, bool) { return false; }
 cudaError_t launch_fields(FieldPhase p, int, const FieldJob*, const Segment*, uint32_t, uint32_t, const FieldJob&, cudaStream_t, uint32_t)
 {
@@ -105,4 +107,5 @@ cudaError_t launch_bitshuffle_flag(const uint32_t*, uint32_t*, uint32_t, uint32_
 cudaError_t launch_decompress_fused(const DecodeArgs&, cudaStream_t) { return fake_call("decompress"); }
 cudaError_t launch_lorenzo_construct(const float*, uint16_t*, uint8_t*, uint32_t, uint32_t, uint32_t, float, cudaStream_t) { return fake_call("construct"); }
 }  // namespace fz
+extern "C" void fake_largest_cluster(uint32_t items) { fz::fake_cluster = items; }
 #endif

@@ -114,3 +114,16 @@ def test_several_at_once(fz, oracle, nd):
     for t in threads:
         t.join()
     assert not bad, bad
+
+
+@pytest.mark.parametrize("nd", [1, 2, 3])
+def test_largest_cluster(fz, nd):
+    """Sixteen items, the range too, in one launch; a range launch from seventeen on."""
+    for items in (16, 17):
+        dims, n = dims_of(nd, items), items * ITEM
+        x, ws = torch.from_numpy(field(n, nd)).cuda(), fz.Workspace(n)
+        ws.enable_timing(16)
+        fz.compress(x, dims, 1e-3, ws=ws)
+        assert ws.kernel_time("k_range_fields")[0] == items - 16
+        assert ws.kernel_time("k_encode_fields")[0] == 1
+        ws.enable_timing(0)

@@ -88,3 +88,39 @@ def test_compress_host_leaves_no_copy_under_way(api, fz, ws):
     st = api.fz_compress_host(ws, x.ctypes.data, x.size, fz.Dims(9000, 1, 1), -1.0, fz.EB_REL, 1, out.ctypes.data, out.size, None, None)
     assert st == fz.INVALID_ARG
     assert api.fake_pending() == 0
+
+
+def compressed(api, fz, ws, items, rel=True):
+    """The launches of one compression of `items` encode items."""
+    n = items * 16384
+    x, out = aligned(n, np.float32), aligned(fz.max_compressed_bytes(n, (n, 1, 1)), np.uint8)
+    api.fake_reset()
+    st = api.fz_compress(ws, x.ctypes.data, n, fz.Dims(n, 1, 1), 1e-3, fz.EB_REL if rel else fz.EB_ABS, 1, out.ctypes.data,
+                         out.size, None, None)
+    assert st == fz.SUCCESS
+    return calls(api)
+
+
+@pytest.mark.parametrize("cluster", [16, 8, 1, 0])
+def test_fields_past_the_largest_cluster_of_the_device(api, fz, ws, cluster):
+    """A cluster that the device cannot place is not launched: such a field takes the other launches."""
+    api.fake_largest_cluster(cluster)
+    try:
+        for items in (1, 8, 9, 16, 17):
+            if items <= cluster:
+                assert compressed(api, fz, ws, items) == ["whole"]
+            else:
+                assert compressed(api, fz, ws, items) == ["range", "encode", "compact"]
+                assert compressed(api, fz, ws, items, rel=False) == ["encode", "compact"]
+        # in a batch: a field of 20 items takes the range of one of 12 ahead unless that is one cluster
+        fields, keep = [], []
+        for items in (20, 12):
+            n = items * 16384
+            x, out = aligned(n, np.float32), aligned(fz.max_compressed_bytes(n, (n, 1, 1)), np.uint8)
+            keep += [x, out]
+            fields.append({"src": x.ctypes.data, "dst": out.ctypes.data, "n": n, "dims": (n, 1, 1), "eb": 1e-3, "dst_capacity": out.size})
+        api.fake_reset()
+        assert api.fz_compress_batch(ws, fz.fields_array(fields), 2, fz.EB_REL, 1, None) == fz.SUCCESS
+        assert calls(api) == ["range", "encode", "compact"] + (["whole"] if cluster >= 12 else ["encode", "compact"])
+    finally:
+        api.fake_largest_cluster(16)
