@@ -448,8 +448,8 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
     J.s2off   = group_sum_l2(ws->max_tiles);
     J.rel    = eb_mode == FZ_EB_REL;
     field_items(L.n, L.nb, a.ntiles, J.rel != 0, J.nr, J.ne, J.nc);
-    const uint32_t clustered = small_items((int)L.ndim);
-    const bool small = J.ne <= clustered, whole = small || (!ra && whole_field_fits((int)L.ndim, J.ne, out_bytes != nullptr));
+    const uint32_t clustered = small_items((int)L.ndim, J.rel != 0);
+    const bool small = J.ne <= clustered, whole = small || (!ra && whole_field_fits((int)L.ndim, J.rel != 0, J.ne, out_bytes != nullptr));
     if (give_up) {
         if (small || !whole || *give_up >= J.ne) return FZ_INVALID_ARG;
         J.give_up = *give_up;
@@ -465,22 +465,22 @@ fz_status fz::compress_impl(fz_workspace* ws, const float* d_in, uint64_t n, fz_
                                               f.dst_capacity, ws->status, Ln, an) == FZ_SUCCESS) {
             uint32_t nr, ne, nc;
             field_items(Ln.n, Ln.nb, an.ntiles, true, nr, ne, nc);
-            if (ne > small_items((int)Ln.ndim)) J.ahead_nr = nr, J.ahead_in = an.in, J.ahead_n = an.n;
+            if (ne > small_items((int)Ln.ndim, true)) J.ahead_nr = nr, J.ahead_in = an.in, J.ahead_n = an.n;
         }
     }
     cudaError_t e = cudaSuccess;
     if (J.nr) {
         KernelTimer t(ws, s, 0);
-        e = launch_fields(FieldPhase::Range, (int)L.ndim, nullptr, nullptr, 0, J.nr, J, s);
+        e = launch_fields(FieldPhase::Range, (int)L.ndim, J.rel != 0, nullptr, nullptr, 0, J.nr, J, s);
     }
     if (e == cudaSuccess) {
         KernelTimer t(ws, s, 1);
         e = whole ? launch_whole_field((int)L.ndim, J, s)
-                  : launch_fields(FieldPhase::Encode, (int)L.ndim, nullptr, nullptr, 0, J.ne, J, s, J.ahead_nr);
+                  : launch_fields(FieldPhase::Encode, (int)L.ndim, J.rel != 0, nullptr, nullptr, 0, J.ne, J, s, J.ahead_nr);
     }
     if (e == cudaSuccess && !whole) {
         KernelTimer t(ws, s, 5);
-        e = launch_fields(FieldPhase::Compact, (int)L.ndim, nullptr, nullptr, 0, J.nc, J, s);
+        e = launch_fields(FieldPhase::Compact, (int)L.ndim, J.rel != 0, nullptr, nullptr, 0, J.nc, J, s);
     }
     if (e != cudaSuccess) return map_err(e);
     if (ra) ra->done = J.ahead_nr != 0;
@@ -797,14 +797,14 @@ fz_status plan_list_compress(fz_workspace* ws, const fz_field* f, uint32_t count
 
 // The batch's compression: one range launch over every field (relative eb), one encode
 // launch per dimensionality present, one compaction launch over every field.
-cudaError_t launch_list_compress(const ListPlan& P, cudaStream_t s)
+cudaError_t launch_list_compress(const ListPlan& P, bool rel, cudaStream_t s)
 {
     const FieldJob none{};
     cudaError_t    e = cudaSuccess;
     for (int k = 0; k < 5 && e == cudaSuccess; ++k) {
         if (!P.total[k]) continue;
         const FieldPhase ph = k == 0 ? FieldPhase::Range : k == 4 ? FieldPhase::Compact : FieldPhase::Encode;
-        e = launch_fields(ph, k >= 1 && k <= 3 ? k : 2, P.jobs, P.seg[k], P.nseg[k], P.total[k], none, s);
+        e = launch_fields(ph, k >= 1 && k <= 3 ? k : 2, rel, P.jobs, P.seg[k], P.nseg[k], P.total[k], none, s);
     }
     return e;
 }
@@ -876,7 +876,7 @@ static fz_status capture_batch(fz_workspace* ws, const fz_field* comp, const fz_
         else {
             // list schedule: the whole compression in a handful of list launches
             if (plan.d_mem) {
-                e = launch_list_compress(plan, cs[0]);
+                e = launch_list_compress(plan, eb_mode == FZ_EB_REL, cs[0]);
                 if (e != cudaSuccess) st = map_err(e);
             }
             // fork: per-field work on parallel branches

@@ -122,6 +122,12 @@ __device__ __forceinline__ float fmin_nan(float a, float b)
     asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
+__device__ __forceinline__ float fmin3_nan(float a, float b, float c)
+{
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 // 1D positions i%4 != 0 store the magnitude only (lorenzo_var.cuh:62).
 __device__ __forceinline__ uint32_t pack_unsigned(float d)
 {

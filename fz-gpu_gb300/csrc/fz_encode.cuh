@@ -6,8 +6,8 @@
 // below 2^24 the reference's float expression (lorenzo_var.cuh:79-295) is exact, so it equals
 // the integer one in any order; while every difference below also fits 16 bits, two elements
 // share one 32-bit word.  The path is taken where that is known before the item (a relative
-// bound: from the field's range) or found while staging it (an absolute bound: from the largest
-// |x * ebx2_r|); other items keep the float path (compute_block).
+// bound: from the field's range) or found while staging it (an absolute bound: from the item's range
+// of x * ebx2_r); other items keep the float path (compute_block).
 //
 // 1. Staging, all threads of the CTA: 16-byte loads, p of each value, and of one difference --
 //    along z in 3D, along y in 2D when rows are too long to stage the row above -- into shared
@@ -89,21 +89,53 @@ __device__ __forceinline__ void quant2(uint64_t v, uint64_t magic, uint32_t& p0,
 __device__ __forceinline__ float lo_of(uint64_t v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float hi_of(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
-// Largest |x r| an item may hold where nothing is known of the field's range: the delta is a
-// signed sum of up to 2^ND values.
+// Whether values of x r of this largest magnitude and within this range stay in 16 bits: a delta at
+// a tile corner is a value itself, along an edge a difference of two, inside a difference of two
+// (2D) or four (3D) such; the partial sums are smaller.  NaN: no.
 template <int ND>
-__device__ __forceinline__ float packed_limit() { return (ND == 1 ? 0.5f : ND == 2 ? 0.25f : 0.125f) * kPackedMax; }
-
-// Whether the whole field stays in 16 bits, from its range: a delta at a tile corner is a value
-// itself, along an edge a difference of two, inside a difference of two (2D) or four (3D)
-// such; the partial sums are smaller.  NaN: no.
+__device__ __forceinline__ bool packed_fits(float peak, float span)
+{
+    return fmax_nan(peak + 1.0f, (ND == 1 ? 1.0f : ND == 2 ? 2.0f : 4.0f) * (span + 2.0f)) < kPackedMax;
+}
+// The whole field, from its range.
 template <int ND>
 __device__ __forceinline__ bool packed_range(const EbInfo& e)
 {
-    const float peak = fmaxf(fabsf(e.vmin), fabsf(e.vmax)) * e.ebx2_r + 1.0f;
-    const float span = (e.vmax - e.vmin) * e.ebx2_r + 2.0f;
-    return peak < kPackedMax && (ND == 1 ? 1.0f : ND == 2 ? 2.0f : 4.0f) * span < kPackedMax;
+    return packed_fits<ND>(fmaxf(fabsf(e.vmin), fabsf(e.vmax)) * e.ebx2_r, (e.vmax - e.vmin) * e.ebx2_r);
 }
+
+// What is known of the values before an item is staged: that they fit, that none is negative too, or
+// nothing.
+enum class Range { Fits, Positive, Unknown };
+
+// Least and largest of a thread's values of x r, both NaN where one is.  Range and peak instead of
+// the peak alone (one instruction a pair of values more): a field far from zero under an absolute
+// bound, 2 to 2.65 at 1e-4 (|x r| up to 13250), was staged, thrown away and encoded in the float
+// path.  fz_compress on GB300, a pass among others: 39200x388 48.9 -> 35.3 us (float path without
+// staging 38), 8192x8192 166 -> 111 (139), 500x500x100 87 -> 50 (72), 501x500x100 113 -> 54 (101); the same fields
+// from zero up at 1e-3 31.0 -> 31.5, 102 -> 99, 46.1 -> 47.0, 49.4 -> 49.7.  An item that does not fit (its range past
+// 16298 quanta in 2D, 8148 in 3D, or codes that overflow) is still staged first, which costs it 10 to 20%:
+// skipping the CTA's next items after such a one, or sampling them, took 1 to 2% from the fields that fit.
+struct Limits {
+    float mn = INFINITY, mx = -INFINITY;
+    __device__ __forceinline__ void add(uint64_t v)
+    {
+        mn = fmin3_nan(mn, lo_of(v), hi_of(v)), mx = fmax3_nan(mx, lo_of(v), hi_of(v));
+    }
+    // Whether the values of all threads of the CTA fit together (one CTA barrier); red: shared, two
+    // words a warp.  f2ord's order holds for numbers only: a NaN goes as an infinity, which does
+    // not fit either.
+    template <int ND>
+    __device__ __forceinline__ bool all_fit(uint32_t (*red)[8]) const
+    {
+        const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+        const uint32_t lo = __reduce_min_sync(kFull, f2ord(mn)), hi = __reduce_max_sync(kFull, f2ord(mx == mx ? mx : INFINITY));
+        if (lane == 0) red[0][wid] = lo, red[1][wid] = hi;
+        __syncthreads();
+        const float l = ord2f(__reduce_min_sync(kFull, red[0][lane & 7u])), h = ord2f(__reduce_max_sync(kFull, red[1][lane & 7u]));
+        return packed_fits<ND>(fmaxf(fabsf(l), fabsf(h)), h - l);
+    }
+};
 
 constexpr uint32_t kStageStep = 256 * 4;  // elements a CTA stages with one group of 4 per thread
 
@@ -156,9 +188,9 @@ struct StageRow {
 // all of them lie inside the field; otherwise groups past its last whole one read that one
 // instead.  kAl: shift % 4 == 0, the neighbours' loads are aligned.  `mine`: whether the last
 // group is stored.
-template <uint32_t kCnt, Diff kDiff, bool kAl, bool kPos, bool kFull>
+template <bool k3D, uint32_t kCnt, Diff kDiff, bool kAl, Range kRange, bool kFull>
 __device__ __forceinline__ void stage_groups(const float* __restrict__ in, uint32_t elast, uint32_t e,
-                                             const StagePlan& p, StageRow& pos, float r, bool track, float& amax,
+                                             const StagePlan& p, StageRow& pos, float r, Limits& lim,
                                              uint8_t* dst, bool mine)
 {
     const uint64_t rr    = pair2(r, r);
@@ -167,6 +199,11 @@ __device__ __forceinline__ void stage_groups(const float* __restrict__ in, uint3
     const float*   src   = in + e;
     const float*   bsrc  = src - p.shift;
     float4         v[kCnt], b[kDiff != Diff::None ? kCnt : 1];
+    // 3D, Diff::Some: the elements without a neighbour, a bit each: the zero in its place is no value of
+    // the item's.  (2D, where the difference is along y and few items hold such elements beside
+    // others, tracks the zeros: the mask there costs 8192x8192 97.6 -> 113 us.)
+    constexpr bool kOwn = k3D && kDiff == Diff::Some && kRange == Range::Unknown;
+    uint32_t       own  = 0;
 #pragma unroll
     for (uint32_t u = 0; u < kCnt; ++u) {
         const uint32_t at = kFull ? u * kStageStep : min(e + u * kStageStep, elast) - e;
@@ -179,6 +216,7 @@ __device__ __forceinline__ void stage_groups(const float* __restrict__ in, uint3
         if (kDiff == Diff::Some && kAl) {
             b[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (pos.row & p.tmask) b[u] = __ldg(reinterpret_cast<const float4*>(bs));
+            else if (kOwn) own |= 15u << (4 * u);
             pos.next(p.shift);
         } else if (kDiff == Diff::Some) {
             const uint32_t left = p.shift - pos.rem;  // elements of the group in this row, if < 4
@@ -188,6 +226,10 @@ __device__ __forceinline__ void stage_groups(const float* __restrict__ in, uint3
             if (left > 1 ? r0 : r1) b[u].y = __ldg(bs + 1);
             if (left > 2 ? r0 : r1) b[u].z = __ldg(bs + 2);
             if (left > 3 ? r0 : r1) b[u].w = __ldg(bs + 3);
+            if (kOwn) {
+                const uint32_t in0 = left >= 4 ? 15u : (1u << left) - 1u;  // the group's elements of this row
+                own |= ((r0 ? 0u : in0) | (r1 ? 0u : 15u & ~in0)) << (4 * u);
+            }
             pos.next(p.shift);
         }
     }
@@ -195,20 +237,21 @@ __device__ __forceinline__ void stage_groups(const float* __restrict__ in, uint3
     for (uint32_t u = 0; u < kCnt; ++u) {
         const uint64_t v0 = scale2(pair2(v[u].x, v[u].y), rr), v1 = scale2(pair2(v[u].z, v[u].w), rr);
         uint32_t       q0, q1, q2, q3;
-        quant2<kPos>(v0, magic, q0, q1);
-        quant2<kPos>(v1, magic, q2, q3);
-        if (!kPos && track) {
-            amax = fmax3_nan(amax, fabsf(lo_of(v0)), fabsf(hi_of(v0)));
-            amax = fmax3_nan(amax, fabsf(lo_of(v1)), fabsf(hi_of(v1)));
+        quant2<kRange == Range::Positive>(v0, magic, q0, q1);
+        quant2<kRange == Range::Positive>(v1, magic, q2, q3);
+        if (kRange == Range::Unknown) {
+            lim.add(v0);
+            lim.add(v1);
         }
         if (kDiff != Diff::None) {
             const uint64_t b0 = scale2(pair2(b[u].x, b[u].y), rr), b1 = scale2(pair2(b[u].z, b[u].w), rr);
             uint32_t       s0, s1, s2, s3;
-            quant2<kPos>(b0, magb, s0, s1);
-            quant2<kPos>(b1, magb, s2, s3);
-            if (!kPos && track) {
-                amax = fmax3_nan(amax, fabsf(lo_of(b0)), fabsf(hi_of(b0)));
-                amax = fmax3_nan(amax, fabsf(lo_of(b1)), fabsf(hi_of(b1)));
+            quant2<kRange == Range::Positive>(b0, magb, s0, s1);
+            quant2<kRange == Range::Positive>(b1, magb, s2, s3);
+            if (kRange == Range::Unknown) {
+                const uint32_t o = own >> (4 * u);
+                lim.add(kOwn ? pair2(o & 1u ? lo_of(v0) : lo_of(b0), o & 2u ? hi_of(v0) : hi_of(b0)) : b0);
+                lim.add(kOwn ? pair2(o & 4u ? lo_of(v1) : lo_of(b1), o & 8u ? hi_of(v1) : hi_of(b1)) : b1);
             }
             // (the bias stays; the upper halves are dropped below)
             q0 -= s0, q1 -= s1, q2 -= s2, q3 -= s3;
@@ -219,15 +262,14 @@ __device__ __forceinline__ void stage_groups(const float* __restrict__ in, uint3
     }
 }
 
-template <Diff kDiff, bool kAl, bool kPos, bool kFull>
-__device__ __forceinline__ float stage_segment(const float* __restrict__ in, uint32_t n, uint32_t base,
-                                               const StagePlan& p, float r, bool track, uint8_t* st)
+template <bool k3D, Diff kDiff, bool kAl, Range kRange, bool kFull>
+__device__ __forceinline__ void stage_segment(const float* __restrict__ in, uint32_t n, uint32_t base,
+                                              const StagePlan& p, float r, Limits& lim, uint8_t* st)
 {
     const uint32_t     elast = (n & ~3u) - 4;
     constexpr uint32_t U    = kDiff != Diff::None ? 4 : 8;  // groups in flight per thread
     constexpr uint32_t kDst = kStageStep / 64 * kStageSlot;
     const uint32_t     t4   = 4 * threadIdx.x;
-    float              amax = 0.0f;
     uint8_t*           dst  = st + 2 * t4 + 8 * (t4 >> 6);
     uint32_t           e    = base + t4;
     if (p.halo && base) {
@@ -236,14 +278,14 @@ __device__ __forceinline__ float stage_segment(const float* __restrict__ in, uin
         uint8_t* dh = dst;
 #pragma unroll 1
         for (; left > kStageStep; left -= min(left, 2 * kStageStep), eh += 2 * kStageStep, dh += 2 * kDst)
-            stage_groups<2, kDiff, kAl, kPos, kFull>(in, elast, eh, p, pos, r, track, amax, dh, t4 + kStageStep < left);
-        if (t4 < left) stage_groups<1, kDiff, kAl, kPos, kFull>(in, elast, eh, p, pos, r, track, amax, dh, true);
+            stage_groups<k3D, 2, kDiff, kAl, kRange, kFull>(in, elast, eh, p, pos, r, lim, dh, t4 + kStageStep < left);
+        if (t4 < left) stage_groups<k3D, 1, kDiff, kAl, kRange, kFull>(in, elast, eh, p, pos, r, lim, dh, true);
     }
     dst += p.halo / 64 * kStageSlot;
     StageRow pos(e, p);
 #pragma unroll 1
     for (uint32_t k = 0; k < kItemCodes / kStageStep; k += U, e += U * kStageStep, dst += U * kDst)
-        stage_groups<U, kDiff, kAl, kPos, kFull>(in, elast, e, p, pos, r, track, amax, dst, true);
+        stage_groups<k3D, U, kDiff, kAl, kRange, kFull>(in, elast, e, p, pos, r, lim, dst, true);
     if (!kFull && (n & 3u)) {
         // the field's last, partial group: the thread that staged another in its place
         const uint32_t i = p.halo + (n & ~3u) - base;
@@ -254,13 +296,13 @@ __device__ __forceinline__ float stage_segment(const float* __restrict__ in, uin
             for (uint32_t k = 0; k < (n & 3u); ++k) {
                 uint32_t unused;
                 uint64_t v = scale2(pair2(__ldg(in + el + k), 0.0f), pair2(r, r));
-                quant2<kPos>(v, pair2(12582912.0f + 32768.0f, 0.0f), q[k], unused);
-                if (!kPos && track) amax = fmax_nan(amax, fabsf(lo_of(v)));
+                quant2<kRange == Range::Positive>(v, pair2(12582912.0f + 32768.0f, 0.0f), q[k], unused);
+                if (kRange == Range::Unknown) lim.add(pair2(lo_of(v), lo_of(v)));
                 if (kDiff == Diff::All || (kDiff == Diff::Some && ((at.rem + k >= p.shift ? at.row + 1 : at.row) & p.tmask))) {
                     uint32_t b;
                     v = scale2(pair2(__ldg(in + el + k - p.shift), 0.0f), pair2(r, r));
-                    quant2<kPos>(v, pair2(12582912.0f, 0.0f), b, unused);
-                    if (!kPos && track) amax = fmax_nan(amax, fabsf(lo_of(v)));
+                    quant2<kRange == Range::Positive>(v, pair2(12582912.0f, 0.0f), b, unused);
+                    if (kRange == Range::Unknown) lim.add(pair2(lo_of(v), lo_of(v)));
                     q[k] -= b;
                 }
             }
@@ -268,27 +310,25 @@ __device__ __forceinline__ float stage_segment(const float* __restrict__ in, uin
                 make_uint2(__byte_perm(q[0], q[1], 0x5410), __byte_perm(q[2], q[3], 0x5410));
         }
     }
-    return amax;
 }
 
 // Staging of elements [base - halo, base + kItemCodes) at st; elements before the field are
 // left unwritten and elements past it hold some other value (no code follows from either).
-// n >= 8, and n >= 2 shift.  Returns the thread's largest
-// |x r| when `track` is set (NaN if one is NaN); kPos: no value is negative, nothing to track.
-template <bool kPos, bool kFull>
-__device__ __forceinline__ float stage_item(const float* __restrict__ in, uint32_t n, uint32_t base,
-                                            const StagePlan& p, float r, bool track, uint8_t* st)
+// n >= 8, and n >= 2 shift.  lim: takes every x r (Range::Unknown).
+template <bool k3D, Range kRange, bool kFull>
+__device__ __forceinline__ void stage_item(const float* __restrict__ in, uint32_t n, uint32_t base,
+                                           const StagePlan& p, float r, Limits& lim, uint8_t* st)
 {
-    if (p.shift == 0) return stage_segment<Diff::None, true, kPos, kFull>(in, n, base, p, r, track, st);
+    if (p.shift == 0) return stage_segment<k3D, Diff::None, true, kRange, kFull>(in, n, base, p, r, lim, st);
     // the rows (planes) the staged elements lie in
     const uint32_t r0 = fdiv(base - (base ? p.halo : 0u), p.dshift), r1 = fdiv(base + kItemCodes - 1, p.dshift);
-    if (r0 == r1 && (r0 & p.tmask) == 0) return stage_segment<Diff::None, true, kPos, kFull>(in, n, base, p, r, track, st);
+    if (r0 == r1 && (r0 & p.tmask) == 0) return stage_segment<k3D, Diff::None, true, kRange, kFull>(in, n, base, p, r, lim, st);
     if ((r0 & p.tmask) && r1 - r0 <= p.tmask - (r0 & p.tmask)) {
-        if (p.shift % 4 == 0) return stage_segment<Diff::All, true, kPos, kFull>(in, n, base, p, r, track, st);
-        return stage_segment<Diff::All, false, kPos, kFull>(in, n, base, p, r, track, st);
+        if (p.shift % 4 == 0) return stage_segment<k3D, Diff::All, true, kRange, kFull>(in, n, base, p, r, lim, st);
+        return stage_segment<k3D, Diff::All, false, kRange, kFull>(in, n, base, p, r, lim, st);
     }
-    if (p.shift % 4 == 0) return stage_segment<Diff::Some, true, kPos, kFull>(in, n, base, p, r, track, st);
-    return stage_segment<Diff::Some, false, kPos, kFull>(in, n, base, p, r, track, st);
+    if (p.shift % 4 == 0) return stage_segment<k3D, Diff::Some, true, kRange, kFull>(in, n, base, p, r, lim, st);
+    return stage_segment<k3D, Diff::Some, false, kRange, kFull>(in, n, base, p, r, lim, st);
 }
 
 // Bits of a where m is set, of b elsewhere.

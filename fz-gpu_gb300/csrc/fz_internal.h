@@ -166,18 +166,18 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 // small_items: kSmallItems, or the largest cluster that the current device can place, where that is
 // smaller (16 is past the portable size of 8; the CTAs of one share a GPC).
 constexpr uint32_t kSmallItems = 16;
-uint32_t    small_items(int nd);
-bool        whole_field_fits(int nd, uint32_t ne, bool waits);
+uint32_t    small_items(int nd, bool rel);
+bool        whole_field_fits(int nd, bool rel, uint32_t ne, bool waits);
 cudaError_t launch_whole_field(int nd, const FieldJob& J, cudaStream_t s);
 
 // Items of each kind for a field of n elements (ntiles scan tiles of shuffle blocks, nb full
 // blocks).
 void field_items(uint32_t n, uint32_t nb, uint32_t ntiles, bool rel, uint32_t& nr, uint32_t& ne, uint32_t& nc);
-// One list launch of `phase` (encode: of dimensionality nd) over `total` items: jobs/segs
+// One list launch of `phase` (encode: of dimensionality nd, under a relative bound or not) over `total` items: jobs/segs
 // device arrays of a batch, or jobs == nullptr and `one` the only field.  The grid is
 // max(total, min_ctas) CTAs, at most one resident wave (min_ctas: an encode launch with
 // range ahead spreads the ahead field's range items over CTAs without encode items).
-cudaError_t launch_fields(FieldPhase phase, int nd, const FieldJob* jobs, const Segment* segs, uint32_t nseg,
+cudaError_t launch_fields(FieldPhase phase, int nd, bool rel, const FieldJob* jobs, const Segment* segs, uint32_t nseg,
                           uint32_t total, const FieldJob& one, cudaStream_t s, uint32_t min_ctas = 0);
 
 struct DecodeArgs {

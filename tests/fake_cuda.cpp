@@ -87,9 +87,9 @@ void field_items(uint32_t n, uint32_t nb, uint32_t ntiles, bool rel, uint32_t& n
     nr = rel ? (uint32_t)cdiv(n, 1024) : 0u, ne = (uint32_t)cdiv(ntiles, 8), nc = (uint32_t)cdiv(nb, 32);
 }
 uint32_t    fake_cluster = 16;
-uint32_t    small_items(int) { return fake_cluster; }
-bool        whole_field_fits(int, uint32_t, bool) { return false; }
-cudaError_t launch_fields(FieldPhase p, int, const FieldJob*, const Segment*, uint32_t, uint32_t, const FieldJob&, cudaStream_t, uint32_t)
+uint32_t    small_items(int, bool) { return fake_cluster; }
+bool        whole_field_fits(int, bool, uint32_t, bool) { return false; }
+cudaError_t launch_fields(FieldPhase p, int, bool, const FieldJob*, const Segment*, uint32_t, uint32_t, const FieldJob&, cudaStream_t, uint32_t)
 {
     return fake_call(p == FieldPhase::Range ? "range" : p == FieldPhase::Encode ? "encode" : "compact");
 }
