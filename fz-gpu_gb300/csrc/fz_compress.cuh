@@ -251,25 +251,88 @@ __device__ __forceinline__ void block2d(const float* __restrict__ in, const Geo&
     ovf |= !(amax < 32768.0f) ? 1u : 0u;
 }
 
+// block2d with the loads kAhead group rows ahead.  Bound by their latency: at the encode kernels' 4 CTAs an
+// SM, fz_compress at a relative 1e-5 on GB300, one row ahead -> two: 8192x8192 210 -> 184 us, 39200x388
+// 54.5 -> 52.1 (with 5 CTAs of 48 registers and one row, before the 16-bit path: 192 and 56.7).  k_compress,
+// pipelined over tiles at 3 CTAs, loses by it (fz_compress_noalloc 39200x388 45.6 -> 50.2) and keeps block2d.
+__device__ __forceinline__ void block2d_ahead(const float* __restrict__ in, const Geo& g, uint32_t base, float r,
+                                              uint32_t lane, uint32_t* sm, uint32_t& ovf)
+{
+    constexpr int kAhead = 2;
+    uint32_t      e0 = base + lane * 4;
+    uint32_t row = fdiv(e0, g.dx), col = e0 - row * g.x;
+    // t = c - n of element base-1, the west neighbour of lane 0's first group
+    float carry = 0.0f;
+    if (lane == 0 && (col & 15u))
+        carry = __fsub_rn(pq(__ldg(in + e0 - 1), r), (row & 15u) ? pq(__ldg(in + e0 - 1 - g.x), r) : 0.0f);
+    float4   v[kAhead], u[kAhead];  // the group row and the row north of it, for kAhead group rows
+    uint32_t c[kAhead];             // column of the first element
+    auto fetch = [&](int k, uint32_t e) {  // at (row, col)
+        v[k] = ldg4(in + e);
+        u[k] = (row & 15u) ? ldg4(in + (e - g.x)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        c[k] = col;
+    };
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+        if (k) advance128(g, e0 + 128 * (k - 1), row, col);
+        fetch(k, e0 + 128 * k);
+    }
+    SwzRot         so(lane);
+    const uint32_t prev = (lane + 31u) & 31u;
+    float          amax = 0.0f;  // max |d| (NaN if any d is NaN)
+#pragma unroll 4
+    for (uint32_t it = 0; it < 16; ++it) {
+        const float4 v0 = v[it % kAhead], u0 = u[it % kAhead];
+        const bool   cin = (c[it % kAhead] & 15u) != 0;
+        if (it + kAhead < 16) {
+            advance128(g, e0 + 128 * (kAhead - 1), row, col);
+            fetch(it % kAhead, e0 + 128 * kAhead);
+        }
+        float t[4];
+        t[0] = __fsub_rn(pq(v0.x, r), pq(u0.x, r));
+        t[1] = __fsub_rn(pq(v0.y, r), pq(u0.y, r));
+        t[2] = __fsub_rn(pq(v0.z, r), pq(u0.z, r));
+        t[3] = __fsub_rn(pq(v0.w, r), pq(u0.w, r));
+        // lane l - 1's t[3]; lane 0 gets lane 31's, its west neighbour one group row on
+        const float rot = __shfl_sync(kFull, t[3], prev);
+        const float tw  = cin ? (lane ? rot : carry) : 0.0f;
+        carry           = rot;
+        float d[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[j] = __fsub_rn(t[j], j ? t[j - 1] : tw);
+        amax = fmax3_nan(amax, fabsf(d[0]), fabsf(d[1]));
+        amax = fmax3_nan(amax, fabsf(d[2]), fabsf(d[3]));
+        *reinterpret_cast<uint2*>(sm + it * 64 + so.x0) =
+            make_uint2(pack_signed_pair(d[0], d[1]), pack_signed_pair(d[2], d[3]));
+        so.next();
+        e0 += 128;
+    }
+    ovf |= !(amax < 32768.0f) ? 1u : 0u;
+}
+
 // A whole 1D shuffle block [base, base+2048) inside the field (c_lorenzo_1d1l,
 // lorenzo_var.cuh:176-214): 256-element Lorenzo blocks with p[-1] = 0 at their start;
 // the code at i%4 == 0 carries its sign, the others the magnitude only (Q2), and the
 // signs of all deltas go to the sidecar words when signw is set.  Lane 0's west
 // neighbour is carried from lane 31 of the previous group row (group rows at odd
-// multiples of 128 continue a 256-element block), and the next row's load is issued
-// before the current one is processed.
+// multiples of 128 continue a 256-element block).  Loads run four group rows ahead: bound by
+// their latency at 4 CTAs an SM (2^25 elements at a relative 1e-5 on GB300, fz_compress: one row ahead
+// 98.9 us, four 94.5, four through a cp.async ring at 3 CTAs 93.8).
 __device__ __forceinline__ void block1d(const float* __restrict__ in, uint32_t base, float r, uint32_t lane,
                                         uint32_t* sm, uint32_t* signw, uint32_t& ovf)
 {
     uint32_t e0    = base + lane * 4;
-    float4   v     = ldg4(in + e0);
+    float4   q[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) q[k] = ldg4(in + e0 + 128 * k);
     float    carry = 0.0f;
     float    amax0 = 0.0f, amax1 = 0.0f;  // max |d| of the signed / magnitude-only positions
     SwzRot         so(lane);
     const uint32_t prev = (lane + 31u) & 31u;
 #pragma unroll 4
     for (uint32_t it = 0; it < 16; ++it) {
-        const float4 vn = it < 15 ? ldg4(in + e0 + 128) : v;
+        const float4 v = q[it % 4];
+        if (it + 4 < 16) q[it % 4] = ldg4(in + e0 + 512);
         const float  p0 = pq(v.x, r), p1 = pq(v.y, r), p2 = pq(v.z, r), p3 = pq(v.w, r);
         const float  rot = __shfl_sync(kFull, p3, prev);  // lane 0: lane 31's, for the next group row
         const float  w   = (e0 & 255u) ? (lane ? rot : carry) : 0.0f;
@@ -292,7 +355,6 @@ __device__ __forceinline__ void block1d(const float* __restrict__ in, uint32_t b
             sv |= __shfl_xor_sync(kFull, sv, 4);
             if ((lane & 7u) == 0) signw[(base >> 5) + it * 4 + (lane >> 3)] = sv;
         }
-        v = vn;
         e0 += 128;
     }
     ovf |= (!(amax0 < 32768.0f) || !(amax1 < 65536.0f)) ? 1u : 0u;
@@ -755,9 +817,9 @@ __device__ __forceinline__ void tail_pads(const CompressArgs& a, uint32_t lane, 
 // Phases A-C for shuffle block t of the field: its codes into the warp's shared buffer
 // `sm` (swizzled), the bit transpose, the shuffled image back into `sm`, the chunk flags
 // as 8 ballots (= bitmap words 8t..8t+7, stored), the chunk count and the overflow bit.
-// Block t == nb (the n mod 2048 tail, never shuffled, fz.cu:173) writes its codes to the
+// kAhead: block2d_ahead for block2d.  Block t == nb (the n mod 2048 tail, never shuffled, fz.cu:173) writes its codes to the
 // sidecar and zero-fills the 16-byte pads of Sections A and C.
-template <int ND>
+template <int ND, bool kAhead>
 __device__ __forceinline__ void compute_block(const CompressArgs& a, const Geo& g, uint32_t t, float r,
                                               uint32_t lane, uint32_t* sm, uint32_t* signw,
                                               uint32_t (&bm)[8], uint32_t& cnt, uint32_t& ovf)
@@ -768,7 +830,8 @@ __device__ __forceinline__ void compute_block(const CompressArgs& a, const Geo& 
         if (ND == 1 && base + kBlockCodes <= g.nl) {
             block1d(a.in, base, r, lane, sm, signw, ovf);
         } else if (ND == 2 && g.al_x && base + kBlockCodes <= g.nl) {
-            block2d(a.in, g, base, r, lane, sm, ovf);
+            if constexpr (kAhead) block2d_ahead(a.in, g, base, r, lane, sm, ovf);
+            else block2d(a.in, g, base, r, lane, sm, ovf);
         } else if (ND == 2 && g.x >= 4 && base + kBlockCodes <= g.nl) {
             block2d_u(a.in, g, base, r, lane, sm, ovf);
         } else if (ND == 3 && g.al_x && base + kBlockCodes <= g.nl) {
@@ -882,7 +945,7 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_compress(const Compr
 
         if (have) {
             uint32_t ovf = 0, cnt = 0;
-            compute_block<ND>(a, g, ct * kCompressWarps + wid, eb.ebx2_r, lane, sm, signw, bm, cnt, ovf);
+            compute_block<ND, false>(a, g, ct * kCompressWarps + wid, eb.ebx2_r, lane, sm, signw, bm, cnt, ovf);
             if (lane == 0) s_cnt[buf][wid] = cnt, s_ovf[buf][wid] = ovf;
             if (threadIdx.x == 0) {  // the CTA's next tile; slot buf^1 (tile k-1) is read only via prev_ct now
                 const Ticket tk = take_ticket(a.ticket, a.epoch, nfetch);
@@ -1126,7 +1189,7 @@ __device__ __forceinline__ void float_block(const FieldJob& J, uint32_t t, float
     g.dx = a.dx, g.dxy = a.dxy, g.al_x = a.al_x, g.al_xy = a.al_xy, g.al_xyx = a.al_xyx;
     uint32_t* signw = (ND == 1 && a.mode == 1) ? reinterpret_cast<uint32_t*>(a.out + a.off_sign) : nullptr;
     uint32_t  bm[8] = {0, 0, 0, 0, 0, 0, 0, 0}, cnt = 0, ovf = 0;
-    compute_block<ND>(a, g, t, r, lane, sm, signw, bm, cnt, ovf);  // warp-uniform t
+    compute_block<ND, true>(a, g, t, r, lane, sm, signw, bm, cnt, ovf);  // warp-uniform t
     if constexpr (!kEmit) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) out.bm[k] = bm[k];
