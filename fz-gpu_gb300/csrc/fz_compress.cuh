@@ -1080,10 +1080,11 @@ __device__ __forceinline__ void locate(const Segment* __restrict__ segs, uint32_
 // so runs differ by at most one item, and keeps kRangeBatch loads per thread in flight.  The
 // running max/min of a thread is carried across its items and folded into the field's
 // accumulators once per field the run touches.
-// The CTA's running max/min go into mm[0..1] (and a non-finite element into *flags and
-// *status) of the field they belong to.
-__device__ __forceinline__ void range_flush(uint32_t* mm, uint32_t* flags, uint32_t* status, float mn, float mx,
-                                            uint32_t nonfinite, uint32_t (*sred)[kCompressWarps])
+// The threads' running max/min and non-finite marks over the CTA, as ordered u32, in `r` (thread 0's).
+struct CtaRange {
+    uint32_t lo, hi, nonfinite;
+};
+__device__ __forceinline__ void range_reduce(float mn, float mx, uint32_t nonfinite, uint32_t (*sred)[kCompressWarps], CtaRange& r)
 {
     // NaN leaves both NaN; -Inf shows in the min, +Inf in the max (the start values +Inf /
     // -Inf of a thread without elements stay on the other side)
@@ -1098,14 +1099,21 @@ __device__ __forceinline__ void range_flush(uint32_t* mm, uint32_t* flags, uint3
     if (lane == 0) sred[0][wid] = f2ord(mn), sred[1][wid] = f2ord(mx), sred[2][wid] = nonfinite;
     __syncthreads();
     if (tid < 32) {
-        const uint32_t a = __reduce_min_sync(kFull, lane < kCompressWarps ? sred[0][lane] : 0xFFFFFFFFu);
-        const uint32_t c = __reduce_max_sync(kFull, lane < kCompressWarps ? sred[1][lane] : 0u);
-        const uint32_t f = __reduce_or_sync(kFull, lane < kCompressWarps ? sred[2][lane] : 0u);
-        if (lane == 0) {
-            atomicMin(mm, a);
-            atomicMax(mm + 1, c);
-            if (f) atomicOr(status, kStatusNonfinite), atomicOr(flags, kStatusNonfinite);
-        }
+        r.lo        = __reduce_min_sync(kFull, lane < kCompressWarps ? sred[0][lane] : 0xFFFFFFFFu);
+        r.hi        = __reduce_max_sync(kFull, lane < kCompressWarps ? sred[1][lane] : 0u);
+        r.nonfinite = __reduce_or_sync(kFull, lane < kCompressWarps ? sred[2][lane] : 0u);
+    }
+}
+// ... into mm[0..1] (and a non-finite element into *flags and *status) of the field they belong to.
+__device__ __forceinline__ void range_flush(uint32_t* mm, uint32_t* flags, uint32_t* status, float mn, float mx,
+                                            uint32_t nonfinite, uint32_t (*sred)[kCompressWarps])
+{
+    CtaRange r;
+    range_reduce(mn, mx, nonfinite, sred, r);
+    if (threadIdx.x == 0) {
+        atomicMin(mm, r.lo);
+        atomicMax(mm + 1, r.hi);
+        if (r.nonfinite) atomicOr(status, kStatusNonfinite), atomicOr(flags, kStatusNonfinite);
     }
     __syncthreads();  // sred before the next flush
 }
@@ -1369,8 +1377,19 @@ __device__ __forceinline__ FieldFinal final_loads(const FieldJob& J)
     return v;
 }
 
-// The header of field J with `total` chunks (and its copy in the mirror, with the status
-// word), the offset table's total, and the control words set for the next call: its range
+// The header of a stream with `total` chunks, and its copy in the mirror, with the status word, so
+// that a caller reads both with one copy; the offset table's total (one thread).
+__device__ __forceinline__ void finish_stream(const CompressArgs& a, const EbInfo& eb, uint32_t flags, uint32_t total, uint32_t status)
+{
+    write_header(a, eb, flags, total, reinterpret_cast<uint4*>(a.mirror));
+    if (a.mirror) a.mirror[16] = status;
+    if (a.boff) {
+        a.boff[a.nb] = total;  // the total closes the offset table; zero its 16-byte pad
+        for (uint32_t k = a.nb + 1; k < (uint32_t)(pad16(4ull * (a.nb + 1)) / 4); ++k) a.boff[k] = 0;
+    }
+}
+
+// finish_stream of field J, and the control words set for the next call: its range
 // and non-finite flag from pre (the range ahead this call's encode launch accumulated, or
 // the empty range), pre reset (one thread; after every encode item of the call).
 __device__ inline void finish_field(const FieldJob& J, uint32_t total, const FieldFinal& v)
@@ -1378,14 +1397,7 @@ __device__ inline void finish_field(const FieldJob& J, uint32_t total, const Fie
     const CompressArgs& a  = J.a;
     FieldCtl*           C  = J.ctl;
     const EbInfo        eb = J.rel ? eb_from_range(ord2f(v.mm0), ord2f(v.mm1), a.eb_rel) : a.ebh;
-    // header and status in the mirror too, so a caller reads both with one copy
-    write_header(a, eb, ((v.flags & kCtlOverflow) ? 1u : 0u) | ((v.flags & kStatusNonfinite) ? 2u : 0u), total,
-                 reinterpret_cast<uint4*>(a.mirror));
-    if (a.mirror) a.mirror[16] = v.status;
-    if (a.boff) {
-        a.boff[a.nb] = total;  // the total closes the offset table; zero its 16-byte pad
-        for (uint32_t k = a.nb + 1; k < (uint32_t)(pad16(4ull * (a.nb + 1)) / 4); ++k) a.boff[k] = 0;
-    }
+    finish_stream(a, eb, ((v.flags & kCtlOverflow) ? 1u : 0u) | ((v.flags & kStatusNonfinite) ? 2u : 0u), total, v.status);
     C->mm[0] = v.pre0, C->mm[1] = v.pre1;
     C->flags = v.pre_flags;
     C->pre[0] = 0xFFFFFFFFu, C->pre[1] = 0u;
@@ -1626,7 +1638,7 @@ __device__ __forceinline__ uint64_t wait_word(bool ok, bool last, uint32_t total
 // tickets, each CTA publishes its chunk count and sums the counts of all items before its own (their
 // CTAs have started, and wait for none after them; a wait gives up after kSpinLimit / 16 rounds).  Past one wave this loses: CTAs that wait hold
 // the memory the next items need, and all wait for the slowest (a persistent form of it took 43.7 us
-// for the 928 items of 39200x388, the encode and compaction launches 23.5 and 8).  Two launches ->
+// for the 929 items of 39200x388, the encode and compaction launches 23.5 and 8).  Two launches ->
 // this one, same measures: 1000x1000 38.8 -> 35.3 / 13.6 -> 11.5, 3600x1800 47.4 -> 42.9 / 21.4 ->
 // 20.2, 128x128x128 40.2 -> 38.4 / 15.1 -> 13.2, 4000000 42.2 -> 40.8 / 16.6 -> 15.3; worst 2000x1500
 // 42.7 -> 40.9 / 15.9 -> 16.0 (184 items: 32 of the 152 SMs have two).  A polling thread per count
@@ -1668,21 +1680,9 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_whole_field(const __
         float          mn = INFINITY, mx = -INFINITY;
         uint32_t       nonfinite = 0;
         for (uint32_t r = r0; r < r1; r += kRangeBatch) range_items(a.in, a.n, r, min(kRangeBatch, r1 - r), mn, mx, nonfinite);
-        nonfinite |= (mn != mn) | (mn == -INFINITY) | (mx == INFINITY);  // (as in range_flush)
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
-            mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
-        }
-        nonfinite = __reduce_or_sync(kFull, nonfinite);
-        if (lane == 0) s_red[0][wid] = f2ord(mn), s_red[1][wid] = f2ord(mx), s_red[2][wid] = nonfinite;
-        __syncthreads();
-        if (wid == 0) {
-            const uint32_t lo = __reduce_min_sync(kFull, lane < kCompressWarps ? s_red[0][lane] : 0xFFFFFFFFu);
-            const uint32_t hi = __reduce_max_sync(kFull, lane < kCompressWarps ? s_red[1][lane] : 0u);
-            const uint32_t nf = __reduce_or_sync(kFull, lane < kCompressWarps ? s_red[2][lane] : 0u);
-            if (lane == 0) s_mine[0] = lo, s_mine[1] = hi, s_mine[2] = nf;
-        }
+        CtaRange mine;
+        range_reduce(mn, mx, nonfinite, s_red, mine);
+        if (tid == 0) s_mine[0] = mine.lo, s_mine[1] = mine.hi, s_mine[2] = mine.nonfinite;
         cluster.sync();
         if (wid == 0) {
             const uint32_t* peer = lane < items ? cluster.map_shared_rank(s_mine, lane) : nullptr;
@@ -1783,12 +1783,7 @@ __global__ void __launch_bounds__(kCompressWarps * 32, 3) k_whole_field(const __
         const uint32_t total = __reduce_add_sync(kFull, pt), ovf = __reduce_or_sync(kFull, peer ? peer[1] : 0u);
         if (lane == 0) {
             const uint32_t st = s_bad ? atomicOr(a.status, kStatusNonfinite) | kStatusNonfinite : a.mirror ? __ldcg(a.status) : 0u;
-            write_header(a, s_eb, (ovf ? 1u : 0u) | (s_bad ? 2u : 0u), total, reinterpret_cast<uint4*>(a.mirror));
-            if (a.mirror) a.mirror[16] = st;
-            if (a.boff) {
-                a.boff[a.nb] = total;  // the total closes the offset table; zero its 16-byte pad
-                for (uint32_t k = a.nb + 1; k < (uint32_t)(pad16(4ull * (a.nb + 1)) / 4); ++k) a.boff[k] = 0;
-            }
+            finish_stream(a, s_eb, (ovf ? 1u : 0u) | (s_bad ? 2u : 0u), total, st);
         }
     }
     if constexpr (kScan) {

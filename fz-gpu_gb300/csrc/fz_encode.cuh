@@ -41,7 +41,7 @@ constexpr uint32_t kItemCodes = 16384;  // elements of an encode item
 // 2 i + 8 (i / 64): the 8-byte pad per 64 elements spreads the lanes' reads, 64 elements apart,
 // over all banks.
 constexpr uint32_t kStageSlot = 136;  // bytes of 64 staged elements
-// Longest row staged as a halo (at most a quarter of an item is staged twice, and 4 CTAs an SM
+// Longest row staged as a halo (about a quarter of an item is staged twice then, and 4 CTAs an SM
 // still fit).  3D rows beyond it take the float path, 2D rows the difference along y while
 // staging.
 constexpr uint32_t kHaloRow = 4096;
