@@ -1,4 +1,4 @@
-// fz_decompress.cu -- decompression kernels (the inverse of fz_compress.cu).
+// fz_decompress.cu -- decompression kernels (the inverse of fz_compress.cuh).
 //
 //   k_decompress1d/2d/3d  fused decode + inverse bitshuffle + inverse Lorenzo, from the
 //              stream straight into the field: each CTA decodes the 64-code groups its

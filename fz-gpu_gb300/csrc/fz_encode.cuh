@@ -23,7 +23,7 @@
 //
 // What bounds it: the float path is bound by instruction issue (3D: 3690 warp instructions per
 // 2048-element block, each value quantised for every stencil role it has); this one issues 1500 (2D
-// 1390), in 41-46% of the cycles: a CTA waits for its item's loads and at the barrier before the
+// 1390), in 38-46% of the cycles: a CTA waits for its item's loads and at the barrier before the
 // images, and the 3-4 CTAs of an SM do not cover each other fully.  Encode launches on GB300, relative bound
 // 1e-3, CUDA events around each launch, float path -> this one: 500x500x100 57.9 -> 33.0 us,
 // 501x500x100 81.7 -> 38.3, 39200x388 26.9 -> 20.8, 8192x8192 97.1 -> 74.5, 3600x1800 16.4 ->
