@@ -1636,7 +1636,8 @@ __device__ __forceinline__ uint64_t wait_word(bool ok, bool last, uint32_t total
 // kScan true, after the range launch, at most one resident wave of items (half a wave when the caller
 // does not wait, whole_field_fits): items are handed out by
 // tickets, each CTA publishes its chunk count and sums the counts of all items before its own (their
-// CTAs have started, and wait for none after them; a wait gives up after kSpinLimit / 16 rounds).  Past one wave this loses: CTAs that wait hold
+// CTAs have started, and wait for none after them; a wait gives up after kSpinLimit / 16 rounds).
+// Past one wave this loses: CTAs that wait hold
 // the memory the next items need, and all wait for the slowest (a persistent form of it took 43.7 us
 // for the 929 items of 39200x388, the encode and compaction launches 23.5 and 8).  Two launches ->
 // this one, same measures: 1000x1000 38.8 -> 35.3 / 13.6 -> 11.5, 3600x1800 47.4 -> 42.9 / 21.4 ->
